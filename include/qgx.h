@@ -40,8 +40,8 @@ typedef struct CUstream_st* qgx_stream_t; /* == cudaStream_t */
 #define QGX_PROPOSAL_LOCAL_FLIP 0    /* quantax.sampler.LocalFlip */
 #define QGX_PROPOSAL_SPIN_EXCHANGE 1 /* quantax.sampler.SpinExchange */
 
-/* diagonal-shifted Cholesky (minnorm_shift_eig): this library's FP64 factorisation (FP64
- * diagonal blocks and triangular solves, every trailing update an exact BF16-digit product on
+/* diagonal-shifted Cholesky (minnorm_shift_eig): this library's FP64 factorisation (64-
+ * column blocks in 60-bit fixed point, every trailing update an exact BF16-digit product on
  * the tensor cores; see qgx_cholesky) */
 #define QGX_SOLVE_SHIFT 0
 #define QGX_SOLVE_PINV 1   /* soft pseudo-inverse via eigh (minnorm_pinv_eig) */
@@ -502,7 +502,7 @@ int qgx_sr_solve(double* S, int64_t np, const float* A, int64_t n, int64_t lda,
  * lower triangle (L[i][j] at A[i lda + j], i >= j); the strict upper triangle keeps the input.
  * Read as column-major, the result is the upper factor U = L^T (A = U^T U) that cuSOLVER's
  * potrs takes with CUBLAS_FILL_MODE_UPPER. 64 x 64 diagonal blocks and their triangular solves
- * run in FP64; every update C -= P P^T (P a 64- or 256-column panel) runs on the tensor cores
+ * run in 60-bit fixed point (each row scaled by the root of its diagonal entry); every update C -= P P^T (P a 64- or 256-column panel) runs on the tensor cores
  * as an exact product of 8 BF16 digit slices per element (row-scaled 57-bit fixed point,
  * integer accumulation exact in FP32), folded in int64 and applied in FP64.
  * info (device int): 0, or the order of the first leading minor that is not positive

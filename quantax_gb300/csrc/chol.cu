@@ -6,10 +6,11 @@
 // holds the matrix by symmetry. Read as column-major, the factor is the upper triangle
 // U = L^T with A = U^T U.
 //
-// FP64 arithmetic runs at about two FMAs per clock per SM on GB300, so only the O(n^2 b) part
-// of the work runs on the FP64 pipe: right-looking, 256-column panels, each factored as four
-// 64-column blocks (potrf of the 64 x 64 diagonal block and the 64-wide triangular solve of
-// every row below it, in FP64). Every update of the form C -= P P^T runs on the tensor cores
+// FP64 arithmetic runs at about two FMAs per clock per SM on GB300 and every FP64 instruction
+// takes 64 clocks, so nothing here runs on the FP64 pipe but the last step of an update:
+// right-looking, 256-column panels, each factored as four 64-column blocks (potrf of the 64 x 64
+// diagonal block and the 64-wide triangular solve of every row below it) in 60-bit fixed point
+// on the integer pipe (qgx_fixed.cuh). Every update of the form C -= P P^T runs on the tensor cores
 // as an exact integer product (the Ozaki scheme: Ozaki, Ogita, Oishi and Rump, "Error-free
 // transformations of matrix multiplication by using fast routines of matrix multiplication and
 // its applications", Numer. Algorithms 59, 2012):
@@ -44,6 +45,7 @@
 #include <vector>
 
 #include "qgx_common.cuh"
+#include "qgx_fixed.cuh"
 #include "qgx_tc.cuh"
 
 namespace qgx {
@@ -65,116 +67,433 @@ constexpr int kOzDLd = kOzN + 1;       // doubles per row of the epilogue's tran
 
 inline int64_t al256(int64_t b) { return (b + 255) / 256 * 256; }
 
+// ---- fixed-point panel ----------------------------------------------------------------------
+// Row r's scale comes from an upper bound on its diagonal entry at the start of the panel,
+// a_rr <= f 2^E (f > 0): set from the matrix, then lowered by each panel's squares.
+struct RowBound {
+  float* f;
+  int* E;
+};
+
+// smallest e with 2^(2e) >= 2 f 2^E: the row's entries of L are below 2^e sqrt(1/2)
+__device__ inline int row_exponent(const RowBound& b, int64_t r) {
+  const float f = fmaxf(b.f[r], 8.6736174e-19f);  // 2^-60: a bound that rounding took to zero
+  const int E = ((__float_as_int(f) >> 23) & 255) - 126 + b.E[r];
+  return (E + 2) >> 1;
+}
+
+// *info: the smallest order of a leading minor found not positive definite (0: none)
+__device__ inline void record_info(int* info, int64_t order) {
+  if (atomicCAS(info, 0, (int)order) != 0) atomicMin(info, (int)order);
+}
+
+__device__ inline double quiet_nan() { return __longlong_as_double(0x7FF8000000000000LL); }
+
+__global__ void diag_bound_kernel(const double* __restrict__ A, int64_t lda, int64_t n, RowBound bound,
+                                  int* __restrict__ info) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  const double a = A[r * lda + r];
+  float f = 0.0f;
+  int E = 0;
+  if (a > 0.0 && dbl_finite(a))
+    f = (float)frexp(a, &E);
+  else
+    record_info(info, r + 1);
+  bound.f[r] = f;
+  bound.E[r] = E;
+}
+
+// the block's factor in fixed point, as the triangular solve reads it
+struct __align__(16) BlockFactor {
+  Fx l[kBlk][kBlk];   // l[k][i] = L_ik 2^-e_i, i > k
+  FxPivot piv[kBlk];  // m = 0: column k is not a number (a pivot at or before it failed)
+};
+
+constexpr float kFullRow = 0.52f;  // a row's squares sum to at most 1/2 (1 + rounding of its bound)
+constexpr float kFxHigh = 4.656612873077393e-10f;  // 2^-31: the unit of Fx::h
+// Work layout of the 64-column chain, potrf_block_kernel and trsm_block_kernel: the columns go in
+// groups of four; lanes are rows, and a warp holds its 32 rows' entries of one group's columns
+// (trsm: of two, w and w + 8). A group's owner scales its four columns one after the other in
+// registers and publishes them in shared memory; after one barrier every warp takes the group's
+// update of its later columns, the next owner first of all. A dead group costs nothing, so the
+// executed multiply-adds are those of the triangle.
+
+// s[e] -= sum over the four columns k of x_k y_k[e], e the four columns of the warp's group;
+// x: entry of the lane's row in column k (stride ldx), y: the group's rows of column k
+__device__ inline void apply_group(const Fx* __restrict__ x, int ldx, const Fx* __restrict__ y, int ldy, int64_t* s1,
+                                   int64_t* s2) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    Fx v = x[k * ldx];
+    v.h = -v.h;
+    v.l = -v.l;
+    const int4 a = *reinterpret_cast<const int4*>(y + k * ldy), b = *reinterpret_cast<const int4*>(y + k * ldy + 2);
+    fx_mad(s1[0], s2[0], v, Fx{a.x, a.y});
+    fx_mad(s1[1], s2[1], v, Fx{a.z, a.w});
+    fx_mad(s1[2], s2[2], v, Fx{b.x, b.y});
+    fx_mad(s1[3], s2[3], v, Fx{b.z, b.w});
+  }
+}
+
+constexpr int kPotrfThreads = 512;
+constexpr int kPotrfLd = kBlk + 2;  // 16-byte rows
+struct PotrfShared {
+  union {
+    double a[kBlk][kBlk + 1];               // the block as read, [row][column]
+    __align__(16) Fx l[kBlk][kPotrfLd];     // the factor, [column][row]
+  };
+  FxPivot piv[kBlk];
+  uint64_t u[kBlk];      // normalised pivots
+  float squares[kBlk];   // of the row's entries so far
+  int e[kBlk];
+  int bad[kBlk];         // row cannot belong to a positive definite matrix
+  int kfail;             // first column whose pivot failed
+};
+
+// the warp's 32 rows (from row0) of the columns k0 .. k0 + 3, all updates taken: scaled and
+// published. PIVOT: the columns' pivots are among these rows and are inverted here (by every
+// lane alike); else they were, a barrier ago.
+template <bool PIVOT>
+__device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, int64_t* s1, int64_t* s2) {
+  const int i = row0 + lane;
+  float squares = sh.squares[i];
+  bool bad = sh.bad[i] != 0;
+  int kfail = sh.kfail;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int k = k0 + e;
+    FxPivot piv;
+    if (PIVOT) {
+      const int src = k - row0;
+      const bool fail = kfail < kBlk || __shfl_sync(0xffffffffu, (int)bad, src) != 0;
+      const int64_t p1 = __shfl_sync(0xffffffffu, s1[e], src), p2 = __shfl_sync(0xffffffffu, s2[e], src);
+      uint64_t u;
+      piv = fx_rsqrt(fail ? -1 : p1, fail ? 0 : p2, &u);
+      if (piv.m == 0) kfail = min(kfail, k);
+      if (lane == 0) {
+        sh.piv[k] = piv;
+        sh.u[k] = u;
+      }
+    } else {
+      piv = sh.piv[k];
+    }
+    bool ok;
+    Fx x = fx_split(fx_scale(s1[e], s2[e], piv, &ok));
+    const float xv = (float)x.h * kFxHigh;
+    const float sq = fmaf(xv, xv, squares);
+    const bool below = i > k && piv.m != 0;
+    bad |= below && (!ok || sq > kFullRow);
+    if (below && !bad)
+      squares = sq;
+    else
+      x = Fx{0, 0};
+    sh.l[k][i] = x;
+    Fx y[4];
+#pragma unroll
+    for (int f = e + 1; f < 4; ++f) {
+      if (PIVOT) {
+        y[f].h = __shfl_sync(0xffffffffu, x.h, k0 + f - row0);
+        y[f].l = __shfl_sync(0xffffffffu, x.l, k0 + f - row0);
+      } else {
+        y[f] = sh.l[k][k0 + f];
+      }
+    }
+    x.h = -x.h;
+    x.l = -x.l;
+#pragma unroll
+    for (int f = e + 1; f < 4; ++f) fx_mad(s1[f], s2[f], x, y[f]);
+  }
+  sh.squares[i] = squares;
+  if (bad) sh.bad[i] = 1;
+  if (PIVOT && lane == 0) sh.kfail = kfail;
+}
+
+// Cholesky of the nb x nb (nb <= 64) diagonal block at (c, c), in place, in fixed point. The
+// first pivot that is not positive makes the remaining columns NaN and is recorded in *info as
+// c + k + 1 (the order of the failing leading minor, as LAPACK and cuSOLVER report it). Eight warps
+// hold rows 0 .. 31, one column group each, and eight rows 32 .. 63, two groups each; the lower
+// rows follow the upper ones by one group. The chain of 64 pivots bounds the kernel (one CTA), so
+// the lower rows' multiply-adds and the stores are kept off the sub-cores that the chain runs on.
+// Measured: 34 us a block (62 us in FP64; of a column's 850 clocks the inverse square root takes
+// 330 and the scaling 140). The factorisation with this kernel and the next: 1.04 ms at n = 1024
+// (1.60 in FP64), 4.6 at 4096 (7.4), 14.0 at 8192 (20.4), 618 at 32768 (668).
+__global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
+                                                                    int nb, RowBound bound,
+                                                                    BlockFactor* __restrict__ out,
+                                                                    int* __restrict__ info) {
+  __shared__ PotrfShared sh;
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  if (t < kBlk) {
+    sh.e[t] = t < nb ? row_exponent(bound, c + t) : 0;
+    sh.bad[t] = 0;
+    sh.squares[t] = 0.0f;
+  }
+  if (t == 0) sh.kfail = kBlk;
+#pragma unroll
+  for (int q = 0; q < kBlk * kBlk / kPotrfThreads; ++q) {
+    const int r = (t >> 6) + q * (kPotrfThreads / kBlk), j = t & 63;
+    sh.a[r][j] = r < nb && j <= r ? A[(c + r) * lda + c + j] : 0.0;
+  }
+  __syncthreads();
+  // warps 0, 1 (mod 4): the upper rows, on two of the SM's four sub-cores; 2, 3: the lower ones
+  const bool lower = (w & 2) != 0;
+  const int g0 = (w >> 2) * 2 + (w & 1), row0 = lower ? 32 : 0, i = row0 + lane;
+  int64_t s1[8], s2[8];  // columns 4 g0 .. and, in the lower rows, 32 + 4 g0 ..
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    s1[q] = s2[q] = 0;
+    if (q >= 4 && !lower) continue;
+    const int j = 4 * g0 + (q & 3) + (q >> 2) * 32;
+    const double a = sh.a[i][j];
+    if (!dbl_finite(a)) sh.bad[i] = 1;
+    // rows past the matrix: a diagonal of 1/4
+    s1[q] = i == j && i >= nb ? 1LL << 60 : fx_from_double(a, sh.e[i] + sh.e[j], 62);
+  }
+  __syncthreads();
+  // column k of 32 rows (of half h) to the matrix and to the triangular solve's copy
+  auto store_column = [&](int k, int h) {
+    const int r = 32 * h + lane;
+    const Fx x = sh.l[k][r];
+    out->l[k][r] = x;
+    if (r >= nb || r < k) return;
+    double v;
+    if (k >= sh.kfail)
+      v = quiet_nan();
+    else if (r == k)
+      v = fx_to_double(fx_sqrt(sh.u[k], sh.piv[k]), sh.e[k] - sh.piv[k].t - 61);
+    else
+      v = fx_to_double(fx_join(x), sh.e[r] - kFxBits);
+    A[(c + r) * lda + c + k] = v;
+    if (r == k) out->piv[k] = sh.piv[k];
+  };
+  auto store_group = [&](int g, int h) {
+#pragma unroll 1
+    for (int e = 0; e < 4; ++e) store_column(4 * g + e, h);
+  };
+#pragma unroll 1
+  for (int step = 0; step < 9; ++step) {
+    const int g = lower ? step - 1 : step;  // the group these rows solve
+    if (g >= 0 && g < 8) {
+      const int k0 = 4 * (g - 1);  // the previous group's first column
+      if (g0 >= g) {
+        if (g > 0) apply_group(&sh.l[k0][i], kPotrfLd, &sh.l[k0][4 * g0], kPotrfLd, s1, s2);
+        if (g0 == g) {
+          if (lower)
+            solve_group<false>(sh, 4 * g, row0, lane, s1, s2);
+          else
+            solve_group<true>(sh, 4 * g, row0, lane, s1, s2);
+        }
+      }
+      if (lower && g > 0) apply_group(&sh.l[k0][i], kPotrfLd, &sh.l[k0][32 + 4 * g0], kPotrfLd, s1 + 4, s2 + 4);
+    }
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (int g = 8; g < 16; ++g) {
+    const int k0 = 4 * (g - 1);
+    if (lower) {
+      if (g0 >= g - 8) {
+        apply_group(&sh.l[k0][i], kPotrfLd, &sh.l[k0][32 + 4 * g0], kPotrfLd, s1 + 4, s2 + 4);
+        if (g0 == g - 8) solve_group<true>(sh, 4 * g, row0, lane, s1 + 4, s2 + 4);
+      }
+    } else if (g0 == g - 8) {
+      store_group(g0, 0);
+    } else if (g0 == ((g - 7) & 7)) {
+      store_group(g0, 1);
+    } else if (g > 8 && g0 == ((g - 6) & 7)) {
+      store_group(g - 1, 1);
+    }
+    __syncthreads();
+  }
+  if (!lower && g0 < 4) store_column(60 + g0, 1);
+  if (t == 0 && sh.kfail < nb) record_info(info, c + sh.kfail + 1);
+}
+
+// The 8 digits of F0 and F1 (|F| <= 2^56), the entries of columns k and k + 1 of a slice row, as
+// BF16 at s + t slice_words for t = 0 .. 7. With 64 added at each of the seven lower places the
+// balanced digits are the 7-bit fields minus 64, the top one the remaining signed part.
+__device__ inline void store_digits(uint32_t* s, int64_t slice_words, int64_t F0, int64_t F1) {
+  const uint64_t F[2] = {(uint64_t)F0 + 0x1020408102040ULL, (uint64_t)F1 + 0x1020408102040ULL};
+#pragma unroll
+  for (int t = 0; t < kSlices; ++t) {
+    uint32_t w[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int d = t == 0 ? (int)((int64_t)F[h] >> 49) : (int)((uint32_t)(F[h] >> (7 * (7 - t))) & 127) - 64;
+      w[h] = __float_as_uint(__int_as_float(0x4B400000 + d) - 12582912.0f);  // (float)d
+    }
+    s[t * slice_words] = __byte_perm(w[0], w[1], 0x7632);  // the high halves: exact in BF16
+  }
+}
+
+// rows [r0, n) of the 64 columns at c: x L_cc^T = a with L_cc the factored diagonal block, in
+// place, and, for the update of the panel's later columns, the rows' digit slices S[t][r][k]
+// (r < n - r0) with exponents ex (S may be NULL). 32 rows per CTA. Bound by the integer pipe at
+// many rows (2016 multiply-adds of three instructions per row), by the chain of 64 scalings at
+// few: 25 us for 8000 rows (56 us in FP64). A row whose squares exceed its bound cannot be completed to a positive definite matrix:
+// its order is recorded and it becomes NaN.
+constexpr int kTrsmThreads = 256, kTrsmWarps = kTrsmThreads / 32;
+constexpr int kTrsmRows = 32;
+struct TrsmShared {
+  BlockFactor f;
+  union {
+    double a[kTrsmRows][kBlk + 1];  // the rows as read
+    Fx x[kBlk][kTrsmRows + 1];      // the solution, [column][row]
+  };
+  float squares[kTrsmRows];
+  int bad[kTrsmRows], nan_row[kTrsmRows];
+  int e[kBlk], er[kTrsmRows];
+};
+
+__device__ inline void trsm_group(TrsmShared& sh, int k0, int lane, int64_t* s1, int64_t* s2) {
+  float squares = sh.squares[lane];
+  bool bad = sh.bad[lane] != 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int k = k0 + e;
+    bool ok;
+    Fx x = fx_split(fx_scale(s1[e], s2[e], sh.f.piv[k], &ok));
+    const float xv = (float)x.h * kFxHigh;
+    squares = fmaf(xv, xv, squares);
+    bad |= !ok || squares > kFullRow;
+    if (bad) x = Fx{0, 0};
+    sh.x[k][lane] = x;
+    x.h = -x.h;
+    x.l = -x.l;
+#pragma unroll
+    for (int f = e + 1; f < 4; ++f) fx_mad(s1[f], s2[f], x, sh.f.l[k][k0 + f]);
+  }
+  sh.squares[lane] = squares;
+  if (bad) sh.bad[lane] = 1;
+}
+
+__global__ void __launch_bounds__(kTrsmThreads) trsm_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
+                                                                  int64_t r0, int64_t n, RowBound bound,
+                                                                  const BlockFactor* __restrict__ factor,
+                                                                  __nv_bfloat16* __restrict__ S, int* __restrict__ ex,
+                                                                  int* __restrict__ info) {
+  extern __shared__ uint8_t smem_raw[];
+  TrsmShared& sh = *reinterpret_cast<TrsmShared*>(smem_raw);
+  static_assert(sizeof(BlockFactor) % 16 == 0, "copied in 16-byte words");
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  const int64_t first = r0 + (int64_t)blockIdx.x * kTrsmRows;
+#pragma unroll
+  for (int e = t; e < (int)(sizeof(BlockFactor) / 16); e += kTrsmThreads)
+    reinterpret_cast<int4*>(&sh.f)[e] = reinterpret_cast<const int4*>(factor)[e];
+  if (t < kBlk) sh.e[t] = row_exponent(bound, c + t);
+  if (t < kTrsmRows) {
+    sh.er[t] = first + t < n ? row_exponent(bound, first + t) : 0;
+    sh.squares[t] = 0.0f;
+    sh.bad[t] = 0;
+    sh.nan_row[t] = 0;
+  }
+#pragma unroll
+  for (int e = t; e < kTrsmRows * kBlk; e += kTrsmThreads) {
+    const int r = e >> 6, j = e & 63;
+    sh.a[r][j] = first + r < n ? A[(first + r) * lda + c + j] : 0.0;  // rows past the matrix solve zeros
+  }
+  __syncthreads();
+  int64_t s1[8], s2[8];  // columns 4 w .. 4 w + 3 and 32 + 4 w ..
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int j = 4 * w + (q & 3) + (q >> 2) * 32;
+    const double a = sh.a[lane][j];
+    if (!dbl_finite(a)) sh.nan_row[lane] = 1;
+    s1[q] = fx_from_double(a, sh.er[lane] + sh.e[j], 62);
+    s2[q] = 0;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int g = 0; g < 8; ++g) {
+    const int k0 = 4 * (g - 1);
+    if (w >= g) {
+      if (g > 0) apply_group(&sh.x[k0][lane], kTrsmRows + 1, &sh.f.l[k0][4 * w], kBlk, s1, s2);
+      if (w == g) trsm_group(sh, 4 * g, lane, s1, s2);
+    }
+    // the owner publishes before it goes on to its second group
+    if (w == g) __syncthreads();
+    if (g > 0) apply_group(&sh.x[k0][lane], kTrsmRows + 1, &sh.f.l[k0][32 + 4 * w], kBlk, s1 + 4, s2 + 4);
+    if (w != g) __syncthreads();
+  }
+#pragma unroll 1
+  for (int g = 8; g < 16; ++g) {
+    const int k0 = 4 * (g - 1);
+    if (w >= g - 8) {
+      apply_group(&sh.x[k0][lane], kTrsmRows + 1, &sh.f.l[k0][32 + 4 * w], kBlk, s1 + 4, s2 + 4);
+      if (w == g - 8) trsm_group(sh, 4 * g, lane, s1 + 4, s2 + 4);
+    }
+    __syncthreads();
+  }
+  // four rows per warp, two neighbouring columns per lane
+  const bool pivots0 = sh.f.piv[2 * lane].m != 0, pivots1 = sh.f.piv[2 * lane + 1].m != 0;
+#pragma unroll 1
+  for (int rl = w; rl < kTrsmRows; rl += kTrsmWarps) {
+    const int64_t rr = first + rl;
+    if (rr >= n) break;
+    const bool bad = sh.bad[rl] != 0, nans = bad || sh.nan_row[rl] != 0;
+    const int e = sh.er[rl];
+    if (bad && lane == 0) record_info(info, rr + 1);
+    const int64_t X0 = fx_join(sh.x[2 * lane][rl]), X1 = fx_join(sh.x[2 * lane + 1][rl]);
+    double* out = A + rr * lda + c + 2 * lane;
+    out[0] = nans || !pivots0 ? quiet_nan() : fx_to_double(X0, e - kFxBits);
+    out[1] = nans || !pivots1 ? quiet_nan() : fx_to_double(X1, e - kFxBits);
+    if (S == nullptr) continue;
+    // every |X| < 2^bits: exponent e + bits - 60, F = X 2^(56 - bits)
+    const uint64_t a0 = X0 < 0 ? 0ULL - (uint64_t)X0 : (uint64_t)X0, a1 = X1 < 0 ? 0ULL - (uint64_t)X1 : (uint64_t)X1;
+    const int bits = __reduce_max_sync(0xffffffffu, 64 - clz64(a0 | a1));
+    const int up = 56 - bits;
+    const int64_t F0 = up >= 0 ? (int64_t)((uint64_t)X0 << up) : (X0 + (1LL << (-up - 1))) >> -up;
+    const int64_t F1 = up >= 0 ? (int64_t)((uint64_t)X1 << up) : (X1 + (1LL << (-up - 1))) >> -up;
+    const int64_t sr = rr - r0;
+    if (lane == 0) ex[sr] = bits == 0 ? 0 : e + bits - kFxBits;
+    store_digits(reinterpret_cast<uint32_t*>(S + sr * kBlk + 2 * lane), (n - r0) * (kBlk / 2), F0, F1);
+  }
+}
+
 // ---- digit slices ---------------------------------------------------------------------------
-// Rows [0, m) of a K-column panel (row r at A + (row0 + r) lda + col0): exponent e_r and the
-// 8 BF16 digit slices S[t][r][k] (slice-major, row stride K). One warp per row.
+// Rows [0, m) of a 256-column panel (row r at A + (row0 + r) lda + col0): exponent e_r and the
+// 8 BF16 digit slices S[t][r][k] (slice-major, row stride 256), and the rows' bounds lowered by
+// the panel's squares. One warp per row, two neighbouring columns per lane and step, integer
+// arithmetic throughout (an FP64 compare or conversion costs 64 clocks per warp): 12 us for 8000
+// rows, 49 MB read and written (61 us with FP64 arithmetic and two-byte stores).
 __global__ void slice_rows_kernel(const double* __restrict__ A, int64_t lda, int64_t row0, int64_t col0, int64_t m,
-                                  int K, __nv_bfloat16* __restrict__ S, int* __restrict__ ex) {
+                                  __nv_bfloat16* __restrict__ S, int* __restrict__ ex, RowBound bound) {
   const int64_t r = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= m) return;  // whole warps
   const double* a = A + (row0 + r) * lda + col0;
-  double mx = 0.0;
-  for (int k = lane; k < K; k += 32) mx = fmax(mx, fabs(a[k]));
+  constexpr int kSteps = kPanel / 64;
+  double v[kSteps][2];
+  uint64_t mx = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  int e = 0;
-  if (mx > 0.0) frexp(mx, &e);  // mx = f 2^e, f in [0.5, 1): every |a_k| < 2^e
+  for (int i = 0; i < kSteps; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      v[i][h] = a[64 * i + 2 * lane + h];
+      const uint64_t b = dbl_bits(v[i][h]) & 0x7FFFFFFFFFFFFFFFULL;
+      mx = b < 0x7FF0000000000000ULL && b > mx ? b : mx;  // NaN and infinities slice as zero
+    }
+  // the exponent with every |a_k| < 2^e; 0 for a zero row
+  const int top = __reduce_max_sync(0xffffffffu, mx == 0 ? -1 : max((int)(mx >> 52), 1));
+  const int e = top < 0 ? 0 : top - 1022;
   if (lane == 0) ex[r] = e;
-  for (int k = lane; k < K; k += 32) {
-    long long F = __double2ll_rn(ldexp(a[k], kFixBits - e));  // exact scaling, |F| <= 2^56
+  float squares = 0.0f;
 #pragma unroll
-    for (int t = kSlices - 1; t >= 1; --t) {
-      const long long d = ((F + 64) & 127) - 64;  // balanced digit in [-64, 64)
-      S[((int64_t)t * m + r) * K + k] = __float2bfloat16_rn((float)d);
-      F = (F - d) >> 7;                           // exact
+  for (int i = 0; i < kSteps; ++i) {
+    int64_t F[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      F[h] = fx_from_double(v[i][h], e, kFixBits);                // |F| <= 2^56
+      const float x = (float)(int)(F[h] >> 26) * 9.3132257e-10f;  // 2^-30
+      squares = fmaf(x, x, squares);
     }
-    S[(int64_t)r * K + k] = __float2bfloat16_rn((float)F);  // |S_0| <= 128
+    store_digits(reinterpret_cast<uint32_t*>(S + r * kPanel + 64 * i + 2 * lane), m * (kPanel / 2), F[0], F[1]);
   }
-}
-
-// ---- FP64 diagonal block and triangular solve -----------------------------------------------
-// Cholesky of the nb x nb (nb <= 64) diagonal block at (c, c), in place. The first pivot that is
-// not positive sets *info = c + k + 1 (the order of the failing leading minor, as LAPACK and
-// cuSOLVER report it); the factorisation carries on with a NaN pivot. 256 threads as a 16 x 16
-// grid over the trailing block (no index division in the update loop); the pivot's inverse
-// square root scales its column.
-__global__ void __launch_bounds__(256) potrf_block_kernel(double* __restrict__ A, int64_t lda, int64_t c, int nb,
-                                                          int* __restrict__ info) {
-  __shared__ double a[kBlk][kBlk + 1];
-  __shared__ double piv[2];  // sqrt and inverse sqrt of the current pivot
-  const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
-  for (int i = ti; i < nb; i += 16)
-    for (int j = tj; j <= i; j += 16) a[i][j] = A[(c + i) * lda + c + j];
-  __syncthreads();
-  for (int k = 0; k < nb; ++k) {
-    if (threadIdx.x == 0) {
-      double d = a[k][k];
-      if (!(d > 0.0)) {
-        atomicCAS(info, 0, (int)(c + k + 1));
-        d = __longlong_as_double(0x7FF8000000000000LL);
-      }
-      const double r = rsqrt(d);
-      piv[0] = d * r;  // sqrt(d)
-      piv[1] = r;
-    }
-    __syncthreads();
-    const double r = piv[1];
-    if (threadIdx.x == 0) a[k][k] = piv[0];
-    for (int i = k + 1 + threadIdx.x; i < nb; i += blockDim.x) a[i][k] *= r;
-    __syncthreads();
-    for (int i = k + 1 + ti; i < nb; i += 16) {
-      const double aik = a[i][k];
-      for (int j = k + 1 + tj; j <= i; j += 16) a[i][j] = fma(-aik, a[j][k], a[i][j]);
-    }
-    __syncthreads();
-  }
-  for (int i = ti; i < nb; i += 16)
-    for (int j = tj; j <= i; j += 16) A[(c + i) * lda + c + j] = a[i][j];
-}
-
-// rows [r0, n) of the 64 columns at c: x L_cc^T = a with L_cc the factored diagonal block, in
-// place (reference BLAS dtrsm 'R','L','T','N' order: scale by the pivot's reciprocal, then
-// update the later columns). Eight lanes per row, lane l holding columns l, l + 8, ..., l + 56:
-// at step k the owner of column k scales it and an 8-lane shuffle hands it to the others, which
-// update their later columns. 16 rows per 128-thread CTA, so even a short panel's rows spread
-// over every SM (the SMs' FP64 pipes bound the work).
-constexpr int kTrsmThreads = 128;
-constexpr int kTrsmRows = kTrsmThreads / 8;
-__global__ void __launch_bounds__(kTrsmThreads) trsm_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
-                                                                  int64_t r0, int64_t n) {
-  __shared__ double l[kBlk][kBlk + 1];
-  __shared__ double dinv[kBlk];
-  for (int e = threadIdx.x; e < kBlk * kBlk; e += blockDim.x) {
-    const int i = e / kBlk, j = e % kBlk;
-    l[i][j] = j <= i ? A[(c + i) * lda + c + j] : 0.0;
-  }
-  for (int i = threadIdx.x; i < kBlk; i += blockDim.x) dinv[i] = 1.0 / A[(c + i) * lda + c + i];
-  __syncthreads();
-  const int sub = threadIdx.x & 7;  // lane within the row's group of eight
-  const int64_t r = r0 + (int64_t)blockIdx.x * kTrsmRows + (threadIdx.x >> 3);
-  const bool live = r < n;  // whole 8-lane groups share a row; dead groups keep shuffling zeros
-  double* row = A + (live ? r : r0) * lda + c;
-  double x[kBlk / 8];
-#pragma unroll
-  for (int q = 0; q < kBlk / 8; ++q) x[q] = live ? row[8 * q + sub] : 0.0;
-#pragma unroll
-  for (int k = 0; k < kBlk; ++k) {
-    const int qk = k >> 3;
-    double xk = 0.0;
-    if (sub == (k & 7)) {
-      x[qk] *= dinv[k];
-      xk = x[qk];
-    }
-    xk = __shfl_sync(0xffffffffu, xk, k & 7, 8);
-#pragma unroll
-    for (int q = 0; q < kBlk / 8; ++q)
-      if (8 * q + sub > k) x[q] = fma(-xk, l[8 * q + sub][k], x[q]);
-  }
-  if (live) {
-#pragma unroll
-    for (int q = 0; q < kBlk / 8; ++q) row[8 * q + sub] = x[q];
-  }
+  squares = warp_sum(squares);
+  // the squares are taken 2^-10 short, far more than the rounding of the float sums: the bound
+  // stays one
+  if (lane == 0) bound.f[row0 + r] -= 0.999f * ldexpf(squares, 2 * e - bound.E[row0 + r]);
 }
 
 // ---- tensor-core update C -= P P^T (lower part) ----------------------------------------------
@@ -471,9 +790,11 @@ int encode_slices(CUtensorMap* map, const __nv_bfloat16* S, int64_t m, int K, in
 
 struct CholWs {
   __nv_bfloat16* s_panel[2];  // 8 x n x 256 digits of a trailing panel (two panels in flight)
-  __nv_bfloat16* s_block;     // 8 x n x 64 digits of a diagonal block's column strip
   int* e_panel[2];            // n row exponents each
+  __nv_bfloat16* s_block;     // 8 x n x 64 digits of the columns below a diagonal block
   int* e_block;               // n row exponents
+  BlockFactor* factor;        // the current diagonal block's
+  RowBound bound;             // n row bounds
 };
 
 int64_t chol_layout(int64_t n, void* base, CholWs* ws) {
@@ -484,27 +805,22 @@ int64_t chol_layout(int64_t n, void* base, CholWs* ws) {
     return o;
   };
   const int64_t o_sp0 = take(kSlices * n * kPanel * 2), o_sp1 = take(kSlices * n * kPanel * 2);
-  const int64_t o_sb = take(kSlices * n * kBlk * 2);
-  const int64_t o_ep0 = take(n * 4), o_ep1 = take(n * 4), o_eb = take(n * 4);
+  const int64_t o_ep0 = take(n * 4), o_ep1 = take(n * 4);
+  const int64_t o_sb = take(kSlices * n * kBlk * 2), o_eb = take(n * 4), o_bf = take(sizeof(BlockFactor));
+  const int64_t o_rf = take(n * 4), o_re = take(n * 4);
   if (base && ws) {
     char* b = static_cast<char*>(base);
     ws->s_panel[0] = reinterpret_cast<__nv_bfloat16*>(b + o_sp0);
     ws->s_panel[1] = reinterpret_cast<__nv_bfloat16*>(b + o_sp1);
-    ws->s_block = reinterpret_cast<__nv_bfloat16*>(b + o_sb);
     ws->e_panel[0] = reinterpret_cast<int*>(b + o_ep0);
     ws->e_panel[1] = reinterpret_cast<int*>(b + o_ep1);
+    ws->s_block = reinterpret_cast<__nv_bfloat16*>(b + o_sb);
     ws->e_block = reinterpret_cast<int*>(b + o_eb);
+    ws->factor = reinterpret_cast<BlockFactor*>(b + o_bf);
+    ws->bound.f = reinterpret_cast<float*>(b + o_rf);
+    ws->bound.E = reinterpret_cast<int*>(b + o_re);
   }
   return off;
-}
-
-// digit slices of the K-column panel at A[row0 .., col0 ..] (m rows)
-int slice_panel(const double* A, int64_t lda, int64_t row0, int64_t col0, int64_t m, int K, __nv_bfloat16* S,
-                int* ex, cudaStream_t st, int64_t* kernels) {
-  if (m <= 0) return QGX_OK;
-  slice_rows_kernel<<<(unsigned)((m + 7) / 8), 256, 0, st>>>(A, lda, row0, col0, m, K, S, ex);
-  ++*kernels;
-  return launch_status();
 }
 
 // C -= P P^T over the region of rows [r0, r0 + m) x columns [q0, q0 + ncols) of A, P the panel
@@ -587,6 +903,10 @@ int chol_f64(double* A, int64_t n, int64_t lda, int* info, int32_t* status, void
   if (status) QGX_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), st));
   QGX_CHECK_CUDA(cudaEventRecord(la->start, st));
   QGX_CHECK_CUDA(cudaStreamWaitEvent(aux, la->start, 0));
+  QGX_CHECK_CUDA(cudaFuncSetAttribute(trsm_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(TrsmShared)));
+  diag_bound_kernel<<<(unsigned)((n + 255) / 256), 256, 0, aux>>>(A, lda, n, ws.bound, info);
+  ++*kernels;
   int64_t k = 0;
   for (int64_t c0 = 0; c0 < n; c0 += kPanel, ++k) {
     const int64_t pe = std::min<int64_t>(c0 + kPanel, n);
@@ -594,27 +914,27 @@ int chol_f64(double* A, int64_t n, int64_t lda, int* info, int32_t* status, void
     // the panel chain
     for (int64_t cj = c0; cj < pe; cj += kBlk) {
       const int nb = (int)std::min<int64_t>(kBlk, n - cj);
-      potrf_block_kernel<<<1, 256, 0, aux>>>(A, lda, cj, nb, info);
+      potrf_block_kernel<<<1, kPotrfThreads, 0, aux>>>(A, lda, cj, nb, ws.bound, ws.factor, info);
       ++*kernels;
       const int64_t rb = cj + kBlk;  // first row below the block
       if (rb >= n) break;
-      trsm_block_kernel<<<(unsigned)((n - rb + kTrsmRows - 1) / kTrsmRows), kTrsmThreads, 0, aux>>>(A, lda, cj, rb,
-                                                                                                      n);
+      trsm_block_kernel<<<(unsigned)((n - rb + kTrsmRows - 1) / kTrsmRows), kTrsmThreads, sizeof(TrsmShared), aux>>>(
+          A, lda, cj, rb, n, ws.bound, ws.factor, rb < pe ? ws.s_block : nullptr, ws.e_block, info);
       ++*kernels;
       if ((rc = launch_status()) != QGX_OK) return rc;
-      if (rb < pe) {  // the block's columns update the rest of the panel (K = 64)
-        if ((rc = slice_panel(A, lda, rb, cj, n - rb, kBlk, ws.s_block, ws.e_block, aux, kernels)) != QGX_OK ||
-            (rc = ozaki_region(A, lda, ws.s_block, ws.e_block, n - rb, rb, kBlk, rb, n - rb, rb, pe - rb, status,
-                               aux, kernels)) != QGX_OK)
-          return rc;
-      }
+      // the block's columns update the rest of the panel (K = 64)
+      if (rb < pe && (rc = ozaki_region(A, lda, ws.s_block, ws.e_block, n - rb, rb, kBlk, rb, n - rb, rb, pe - rb,
+                                        status, aux, kernels)) != QGX_OK)
+        return rc;
     }
     if (pe >= n) break;
     // the panel's trailing update (K = 256): the strip on the internal stream, the rest on st
     const int b = (int)(k & 1);
     const int64_t ms = n - pe, pe2 = std::min<int64_t>(pe + kPanel, n);
-    if ((rc = slice_panel(A, lda, pe, c0, ms, kPanel, ws.s_panel[b], ws.e_panel[b], aux, kernels)) != QGX_OK)
-      return rc;
+    slice_rows_kernel<<<(unsigned)((ms + 7) / 8), 256, 0, aux>>>(A, lda, pe, c0, ms, ws.s_panel[b], ws.e_panel[b],
+                                                                ws.bound);
+    ++*kernels;
+    if ((rc = launch_status()) != QGX_OK) return rc;
     // the strip updates the next panel's columns, which the previous panel's rest update (on st)
     // also updates: both read-modify-write the same entries, so the strip waits for it
     if (k >= 1) QGX_CHECK_CUDA(cudaStreamWaitEvent(aux, la->rest_done[(k - 1) & 1], 0));
