@@ -26,16 +26,8 @@
 // The products with t + u >= 8 are dropped: with the digits' own truncation the update's error
 // is a few 2^-56 K 2^(e_i + e_j), below FP64's own rounding of a K-term dot product.
 //
-// The tensor-core kernel: one CTA per 128 x 32 tile of C on or below the diagonal, two CTAs
-// per SM (one CTA's epilogue overlaps the other's MMAs). Warp 4 loads the 8 digit slices of the
-// tile's 128 A rows and 32 B rows, 32 K-elements per stage (3D TMA box, 64-byte swizzle, one
-// stage); warp 5 issues, per 16-element K step, one tcgen05.mma per A slice t (M 128,
-// N = 32 (8 - t), K 16, BF16 -> FP32) against the B slices 0 .. 7 - t side by side, so the
-// eight 32-column level accumulators (256 TMEM columns) each collect their level's products;
-// warps 0-3 read the levels back and fold them in int64 into a shared-memory tile of FP64
-// deltas, and all six warps apply the update to C in coalesced rows. Every mbarrier wait is
-// bounded (2 s); a wait that runs out records QGX_ERR_TIMEOUT, the CTA frees its TMEM and
-// leaves C alone.
+// The tensor-core kernel (ozaki_syrk_kernel) takes 128 x 64 tiles of C, one CTA per SM and a few
+// tiles per CTA; the digits are stored as the shared-memory image of its operands.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -55,15 +47,25 @@ constexpr int kPanel = 256;                     // columns of one tensor-core tr
 constexpr int kBlk = 64;                        // columns of one FP64 diagonal block
 constexpr int kSlices = 8;                      // BF16 digits per element
 constexpr int kFixBits = 56;                    // kSlices * 7 fraction bits of the sliced rows
-constexpr int kOzM = 128, kOzN = 32, kOzKB = 32;  // tile rows, tile columns, K per stage
-constexpr int kOzStages = 1;  // two CTAs per SM: one CTA's epilogue overlaps the other's MMAs
-constexpr int kOzABytes = kSlices * kOzM * kOzKB * 2;  // 64 KB
-constexpr int kOzBBytes = kSlices * kOzN * kOzKB * 2;  // 16 KB
+constexpr int kOzM = 128, kOzN = 64, kOzKB = 32;  // tile rows, tile columns, K per stage
+constexpr int kOzStages = 2;
+constexpr int kOzRowBytes = kOzKB * 2;                         // one operand row of a stage
+constexpr int kOzABytes = kSlices * kOzM * kOzRowBytes;        // 64 KB
+constexpr int kOzBBytes = kSlices * kOzN * kOzRowBytes;        // 32 KB
 constexpr int kOzStageBytes = kOzABytes + kOzBBytes;
-constexpr int kOzThreads = 192;
-constexpr size_t kOzSmem = 1024 + (size_t)kOzStages * kOzStageBytes + 256;
-constexpr uint32_t kOzTmemCols = kSlices * kOzN;  // eight 32-column FP32 level accumulators
-constexpr int kOzDLd = kOzN + 1;       // doubles per row of the epilogue's transpose tile
+constexpr int kOzEpiWarps = 8;                                 // epilogue warps; then producer, MMA issuer
+constexpr int kOzThreads = 32 * (kOzEpiWarps + 2);
+constexpr int kOzTurn = 8, kOzTurnLd = kOzTurn + 1;            // columns per turn through the transpose buffers
+constexpr int kOzTurnBytes = kOzEpiWarps * 32 * kOzTurnLd * 8;
+constexpr size_t kOzSmem = 1024 + (size_t)kOzStages * kOzStageBytes + kOzTurnBytes + 256;
+constexpr uint32_t kOzTmemCols = kSlices * kOzN;               // eight 64-column FP32 level accumulators
+constexpr int kOzGroup = 8;                                    // row tiles per rasterisation group
+
+// Digit slices are stored as the operand images of the update's stages: [128-row block][32-column
+// block][slice][row][64 bytes], the 16-byte chunks of a row swizzled as the 64-byte swizzle of the
+// MMA descriptors has them, so that a stage's A operand is one contiguous 64 KB copy and its B
+// operand (a 64-row half) eight of 4 KB.
+inline int64_t slice_rows(int64_t n) { return (n + kOzM - 1) / kOzM * kOzM; }
 
 inline int64_t al256(int64_t b) { return (b + 255) / 256 * 256; }
 
@@ -310,10 +312,12 @@ __global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __re
   if (t == 0 && sh.kfail < nb) record_info(info, c + sh.kfail + 1);
 }
 
-// The 8 digits of F0 and F1 (|F| <= 2^56), the entries of columns k and k + 1 of a slice row, as
-// BF16 at s + t slice_words for t = 0 .. 7. With 64 added at each of the seven lower places the
-// balanced digits are the 7-bit fields minus 64, the top one the remaining signed part.
-__device__ inline void store_digits(uint32_t* s, int64_t slice_words, int64_t F0, int64_t F1) {
+// The 8 digits of F0 and F1 (|F| <= 2^56), columns k and k + 1 (k even) of slice row r, into the
+// slices of kblocks 32-column blocks. With 64 added at each of the seven lower places the balanced
+// digits are the 7-bit fields minus 64, the top one the remaining signed part.
+__device__ inline void store_digits(uint8_t* S, int kblocks, int64_t r, int k, int64_t F0, int64_t F1) {
+  const int row = (int)(r & (kOzM - 1)), chunk = ((k >> 3) & 3) ^ ((row >> 1) & 3);
+  uint8_t* s = S + ((r / kOzM) * kblocks + (k >> 5)) * (int64_t)kOzABytes + row * kOzRowBytes + chunk * 16 + (k & 7) * 2;
   const uint64_t F[2] = {(uint64_t)F0 + 0x1020408102040ULL, (uint64_t)F1 + 0x1020408102040ULL};
 #pragma unroll
   for (int t = 0; t < kSlices; ++t) {
@@ -323,13 +327,14 @@ __device__ inline void store_digits(uint32_t* s, int64_t slice_words, int64_t F0
       const int d = t == 0 ? (int)((int64_t)F[h] >> 49) : (int)((uint32_t)(F[h] >> (7 * (7 - t))) & 127) - 64;
       w[h] = __float_as_uint(__int_as_float(0x4B400000 + d) - 12582912.0f);  // (float)d
     }
-    s[t * slice_words] = __byte_perm(w[0], w[1], 0x7632);  // the high halves: exact in BF16
+    // the high halves: exact in BF16
+    *reinterpret_cast<uint32_t*>(s + t * (kOzM * kOzRowBytes)) = __byte_perm(w[0], w[1], 0x7632);
   }
 }
 
 // rows [r0, n) of the 64 columns at c: x L_cc^T = a with L_cc the factored diagonal block, in
-// place, and, for the update of the panel's later columns, the rows' digit slices S[t][r][k]
-// (r < n - r0) with exponents ex (S may be NULL). 32 rows per CTA. Bound by the integer pipe at
+// place, and, for the update of the panel's later columns, the rows' digit slices S (slice row r -
+// r0) with exponents ex (S may be NULL). 32 rows per CTA. Bound by the integer pipe at
 // many rows (2016 multiply-adds of three instructions per row), by the chain of 64 scalings at
 // few: 25 us for 8000 rows (56 us in FP64). A row whose squares exceed its bound cannot be completed to a positive definite matrix:
 // its order is recorded and it becomes NaN.
@@ -371,7 +376,7 @@ __device__ inline void trsm_group(TrsmShared& sh, int k0, int lane, int64_t* s1,
 __global__ void __launch_bounds__(kTrsmThreads) trsm_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
                                                                   int64_t r0, int64_t n, RowBound bound,
                                                                   const BlockFactor* __restrict__ factor,
-                                                                  __nv_bfloat16* __restrict__ S, int* __restrict__ ex,
+                                                                  uint8_t* __restrict__ S, int* __restrict__ ex,
                                                                   int* __restrict__ info) {
   extern __shared__ uint8_t smem_raw[];
   TrsmShared& sh = *reinterpret_cast<TrsmShared*>(smem_raw);
@@ -447,18 +452,17 @@ __global__ void __launch_bounds__(kTrsmThreads) trsm_block_kernel(double* __rest
     const int64_t F1 = up >= 0 ? (int64_t)((uint64_t)X1 << up) : (X1 + (1LL << (-up - 1))) >> -up;
     const int64_t sr = rr - r0;
     if (lane == 0) ex[sr] = bits == 0 ? 0 : e + bits - kFxBits;
-    store_digits(reinterpret_cast<uint32_t*>(S + sr * kBlk + 2 * lane), (n - r0) * (kBlk / 2), F0, F1);
+    store_digits(S, kBlk / kOzKB, sr, 2 * lane, F0, F1);
   }
 }
 
 // ---- digit slices ---------------------------------------------------------------------------
 // Rows [0, m) of a 256-column panel (row r at A + (row0 + r) lda + col0): exponent e_r and the
-// 8 BF16 digit slices S[t][r][k] (slice-major, row stride 256), and the rows' bounds lowered by
-// the panel's squares. One warp per row, two neighbouring columns per lane and step, integer
+// 8 BF16 digit slices S, and the rows' bounds lowered by the panel's squares. One warp per row, two neighbouring columns per lane and step, integer
 // arithmetic throughout (an FP64 compare or conversion costs 64 clocks per warp): 12 us for 8000
 // rows, 49 MB read and written (61 us with FP64 arithmetic and two-byte stores).
 __global__ void slice_rows_kernel(const double* __restrict__ A, int64_t lda, int64_t row0, int64_t col0, int64_t m,
-                                  __nv_bfloat16* __restrict__ S, int* __restrict__ ex, RowBound bound) {
+                                  uint8_t* __restrict__ S, int* __restrict__ ex, RowBound bound) {
   const int64_t r = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= m) return;  // whole warps
@@ -488,7 +492,7 @@ __global__ void slice_rows_kernel(const double* __restrict__ A, int64_t lda, int
       const float x = (float)(int)(F[h] >> 26) * 9.3132257e-10f;  // 2^-30
       squares = fmaf(x, x, squares);
     }
-    store_digits(reinterpret_cast<uint32_t*>(S + r * kPanel + 64 * i + 2 * lane), m * (kPanel / 2), F[0], F[1]);
+    store_digits(S, kPanel / kOzKB, r, 64 * i + 2 * lane, F[0], F[1]);
   }
   squares = warp_sum(squares);
   // the squares are taken 2^-10 short, far more than the rounding of the float sums: the bound
@@ -520,11 +524,11 @@ __device__ inline void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
 
-__device__ inline void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+// bulk copy of bytes (a multiple of 16) from global to shared memory, both 16-byte aligned
+__device__ inline void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], "
-      "[%2];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
 
@@ -541,38 +545,56 @@ __device__ inline void tmem_ld_16cols_nowait(uint32_t taddr, uint32_t (&r)[16]) 
 
 __device__ inline void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// level l's integer, scaled to 2^(38 - 7 l) (levels 6 and 7 rounded to the nearest 2^-38)
-template <int L>
-__device__ inline long long level_term(int v) {
-  constexpr int s = 38 - 7 * L;
-  if constexpr (s >= 0) {
-    return (long long)v << s;
-  } else {
-    return ((long long)v + (1LL << (-s - 1))) >> (-s);
+// Tile `index` of the lower part of an m x ncols region whose diagonal starts at its corner, in
+// groups of kOzGroup row tiles, column by column inside a group, so that the tiles in flight share
+// operand blocks in L2. False for the enumeration's tiles above the diagonal (among a group's last
+// columns), which the caller skips.
+__device__ inline bool oz_tile(int64_t index, int64_t m, int64_t ncols, int64_t* bi, int64_t* bj) {
+  const int64_t nr = (m + kOzM - 1) / kOzM, nc = (ncols + kOzN - 1) / kOzN;
+  for (int64_t g = 0; g * kOzGroup < nr; ++g) {
+    const int64_t rows = min((int64_t)kOzGroup, nr - g * kOzGroup);
+    const int64_t cols = min(nc, 2 * (g * kOzGroup + rows));
+    if (index < rows * cols) {
+      *bi = g * kOzGroup + index % rows;
+      *bj = index / rows;
+      return *bj <= 2 * *bi + 1;
+    }
+    index -= rows * cols;
   }
+  return false;
 }
 
-// 2^x for any exponent an FP64 update can take
-__device__ inline double pow2(int x) {
-  if (x >= -1022 && x <= 1023) return __hiloint2double((x + 1023) << 20, 0);
-  return ldexp(1.0, x);
-}
-
-// C[i][j] -= sum_k P[a0 + i][k] P[b0 + j][k] for the m x ncols region at C (ldc), where slice
-// row r is the panel's row r; only entries with a0 + i >= b0 + j (on or below the diagonal of the
-// whole matrix) are updated
-__global__ void __launch_bounds__(kOzThreads, 2)
-    ozaki_syrk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                      const int* __restrict__ ex, int64_t m, int64_t ncols, int a0, int b0, int nkb,
-                      double* __restrict__ C, int64_t ldc, int32_t* __restrict__ status) {
-  const int64_t row0 = (int64_t)blockIdx.x * kOzM, col0 = (int64_t)blockIdx.y * kOzN;
-  if (a0 + row0 + kOzM - 1 < b0 + col0) return;  // the tile lies above the diagonal: nothing to update
+// C[i][j] -= sum_k P[i][k] P[j][k] for i >= j in the m x ncols region at C (ldc), slice row
+// off + i (off a multiple of 128) being P's row i; kblocks 32-column blocks of P.
+//
+// Warps 0-7: epilogue; warp 8: the producer; warp 9: the MMA issuer. Per 16-element K step the
+// issuer multiplies each A slice t (M 128) with the B slices u = 0 .. 7 - t, which lie side by side
+// in shared memory, so D's 64-column block u is S_t S_u^T and lands in the accumulator of level
+// t + u: levels t .. 7 are one contiguous range of N = 64 (8 - t) columns, taken in instructions of
+// at most 256. Every level sum stays an integer below 2^24, so the FP32 accumulation is exact in
+// any order. The eight accumulators fill the tensor memory; the epilogue warps (warp w: TMEM lanes
+// 32 (w mod 4) .., columns 32 (w / 4) ..) first fold all levels into registers, which frees it for
+// the next tile's MMAs, and update C beside those, through transpose buffers of eight columns.
+//
+// Why 128 x 64: the MMAs of a K step take 1152 clocks at the tensor cores' rate and its operands are
+// 48 KB, 42 bytes a clock and SM out of L2 (71 for 128 x 32 tiles). Why a few tiles per CTA and not
+// a persistent grid: the panel chain of the look-ahead runs beside this kernel and gets an SM only
+// when a CTA ends. Measured: 1.67 ms for the 15872-row update of a 16384 factorisation, tensor pipe
+// 59% (31.5% for 128 x 32 tiles, two CTAs per SM, single 80 KB stages, 36 products of N = 32 ..
+// 256); the rest is the drain of the accumulators between tiles and the first and last tile of a
+// CTA. The factorisation at n = 32768: 342 ms, 617 before.
+__global__ void __launch_bounds__(kOzThreads, 1)
+    ozaki_syrk_kernel(const uint8_t* __restrict__ S, const int* __restrict__ ex, int kblocks, int off, int64_t m,
+                      int64_t ncols, double* __restrict__ C, int64_t ldc, int64_t tiles, int per_cta,
+                      int32_t* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kOzStages * kOzStageBytes);
+  double* turn = reinterpret_cast<double*>(smem + kOzStages * kOzStageBytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kOzStages * kOzStageBytes + kOzTurnBytes);
   uint64_t* empty = full + kOzStages;
   uint64_t* acc_full = empty + kOzStages;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint64_t* acc_empty = acc_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
   volatile int* fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -582,6 +604,7 @@ __global__ void __launch_bounds__(kOzThreads, 2)
       mbar_init(&empty[s], 1);
     }
     mbar_init(acc_full, 1);
+    mbar_init(acc_empty, kOzEpiWarps);
     *fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -596,202 +619,159 @@ __global__ void __launch_bounds__(kOzThreads, 2)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  const int64_t first = blockIdx.x * (int64_t)per_cta, last = min(tiles, first + per_cta);
+  int64_t bi = 0, bj = 0;
 
-  int issued = 0;  // producer: stage loads issued
-  if (warp == 4) {
+  if (warp == kOzEpiWarps) {
     if (lane == 0) {
-      for (int kb = 0; kb < nkb && !*fail; ++kb, ++issued) {
-        const int s = kb % kOzStages;
-        const uint32_t ph = (uint32_t)((kb / kOzStages) & 1);
-        if (!mbar_wait(&empty[s], ph ^ 1u)) {
-          *fail = 1;
-          break;
+      int it = 0;  // stage loads issued
+      for (int64_t tile = first; tile < last && !*fail; ++tile) {
+        if (!oz_tile(tile, m, ncols, &bi, &bj)) continue;
+        const uint8_t* a = S + (off / kOzM + bi) * kblocks * (int64_t)kOzABytes;
+        const int64_t br = off / kOzN + bj;  // 64-row half blocks
+        const uint8_t* b = S + (br >> 1) * kblocks * (int64_t)kOzABytes + (br & 1) * (kOzN * kOzRowBytes);
+        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+          const int s = it % kOzStages;
+          if (!mbar_wait(&empty[s], (uint32_t)((it / kOzStages) & 1) ^ 1u)) {
+            *fail = 1;
+            break;
+          }
+          uint8_t* dst = smem + s * kOzStageBytes;
+          mbar_expect_tx(&full[s], kOzStageBytes);
+          bulk_load(dst, a + kb * (int64_t)kOzABytes, kOzABytes, &full[s]);
+#pragma unroll
+          for (int t = 0; t < kSlices; ++t)
+            bulk_load(dst + kOzABytes + t * (kOzN * kOzRowBytes),
+                      b + kb * (int64_t)kOzABytes + t * (kOzM * kOzRowBytes), kOzN * kOzRowBytes, &full[s]);
         }
-        uint8_t* a = smem + s * kOzStageBytes;
-        mbar_expect_tx(&full[s], kOzStageBytes);
-        tma_load_3d(a, &map_a, &full[s], kb * kOzKB, a0 + (int)row0, 0);
-        tma_load_3d(a + kOzABytes, &map_b, &full[s], kb * kOzKB, b0 + (int)col0, 0);
       }
+      if (*fail)  // no copy may land in shared memory after the CTA has left: wait (bounded)
+        for (int k = max(0, it - kOzStages); k < it; ++k)
+          mbar_wait(&full[k % kOzStages], (uint32_t)((k / kOzStages) & 1));
     }
-  } else if (warp == 5) {
+  } else if (warp == kOzEpiWarps + 1) {
     if (lane == 0) {
-      for (int kb = 0; kb < nkb && !*fail; ++kb) {
-        const int s = kb % kOzStages;
-        const uint32_t ph = (uint32_t)((kb / kOzStages) & 1);
-        if (!mbar_wait(&full[s], ph)) {
+      int it = 0, done = 0;  // stages consumed, tiles issued
+      for (int64_t tile = first; tile < last && !*fail; ++tile) {
+        if (!oz_tile(tile, m, ncols, &bi, &bj)) continue;
+        if (done > 0 && !mbar_wait(acc_empty, (uint32_t)(done - 1) & 1u)) {
           *fail = 1;
           break;
         }
         tc_fence_after();
-        const uint32_t base = smem_u32(smem + s * kOzStageBytes);
-#pragma unroll 1
-        for (int kk = 0; kk < kOzKB / 16; ++kk) {  // 32 bytes of K per instruction
-          // one MMA per A slice t: B is the slices u = 0 .. 7 - t of the column rows, contiguous
-          // in shared memory (slice u at rows kOzN u ..), so D's column block u is S_t S_u^T and
-          // lands in the accumulator of level t + u (columns kOzN (t + u) ..): levels t .. 7
-          // are one contiguous N = kOzN (8 - t) range. Every level sum stays an integer below
-          // 2^24, so the FP32 accumulation is exact in any order.
-          const uint64_t db = desc_sw64(base + kOzABytes + kk * 32);
-#pragma unroll
-          for (int t = 0; t < kSlices; ++t) {
-            const uint64_t da = desc_sw64(base + t * (kOzM * kOzKB * 2) + kk * 32);
-            mma_bf16(tmem + (uint32_t)(kOzN * t), da, db, oz_idesc(kOzN * (kSlices - t)),
-                     (kb == 0 && kk == 0 && t == 0) ? 0u : 1u);
+        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+          const int s = it % kOzStages;
+          if (!mbar_wait(&full[s], (uint32_t)((it / kOzStages) & 1))) {
+            *fail = 1;
+            break;
           }
-        }
-        mma_commit(&empty[s]);
-      }
-      mma_commit(acc_full);  // also after a failed wait: tracks every MMA issued so far
-    }
-  }
-
-  // epilogue warps 0..3: fold the eight levels of each row (TMEM lane) into FP64 deltas
-  double* dt = reinterpret_cast<double*>(smem);  // 128 x 65 doubles over the (finished) stages
-  const int q = warp & 3;
-  if (warp < 4) {
-    // while the MMAs run: pull this tile's rows of C into L2 for the read-modify-write below
-    for (int rr = q; rr < kOzM; rr += 4) {
-      const int64_t i = row0 + rr;
-      if (i >= m) break;
-      // lanes 0-3: the cache lines holding columns 16 lane .. of the row (every address lies in C)
-      if (lane < kOzN / 16 && col0 + 16 * lane < ncols)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(C + i * ldc + col0 + 16 * lane));
-    }
-    if (!mbar_wait(acc_full, 0)) *fail = 1;
-    if (!*fail) {
-      tc_fence_after();
-      const int rl = 32 * q + lane;
-      const uint32_t lane_addr = tmem + ((uint32_t)(32 * q) << 16);
+          tc_fence_after();
+          const uint32_t base = smem_u32(smem + s * kOzStageBytes);
 #pragma unroll 1
-      for (int g = 0; g < kOzN / 16; ++g) {
-        long long v[16];
-        // four levels in flight behind one wait, twice
+          for (int kk = 0; kk < kOzKB / 16; ++kk) {  // 32 bytes of K per instruction
+#pragma unroll
+            for (int t = 0; t < kSlices; ++t) {
+              const uint64_t da = desc_sw64(base + t * (kOzM * kOzRowBytes) + kk * 32);
+#pragma unroll
+              for (int u = 0; u < kSlices - t; u += 4) {
+                const int n = kOzN * (kSlices - t - u < 4 ? kSlices - t - u : 4);
+                const uint64_t db = desc_sw64(base + kOzABytes + u * (kOzN * kOzRowBytes) + kk * 32);
+                mma_bf16(tmem + (uint32_t)(kOzN * (t + u)), da, db, oz_idesc(n), (kb == 0 && kk == 0 && t == 0) ? 0u : 1u);
+              }
+            }
+          }
+          mma_commit(&empty[s]);
+        }
+        mma_commit(acc_full);  // also after a failed wait: tracks every MMA issued so far
+        if (*fail) mbar_wait(acc_full, (uint32_t)done & 1u);
+        ++done;
+      }
+    }
+  } else {
+    const int q = warp & 3, cols0 = 32 * (warp >> 2);
+    double* tr = turn + warp * 32 * kOzTurnLd;
+    int done = 0;
+    for (int64_t tile = first; tile < last && !*fail; ++tile) {
+      if (!oz_tile(tile, m, ncols, &bi, &bj)) continue;
+      const int64_t row0 = bi * kOzM + 32 * q, col0 = bj * kOzN + cols0;
+      const int64_t i = row0 + lane;
+      const int ei = i < m ? ex[off + i] : 0;
+      const int ej = col0 + lane < ncols ? ex[off + col0 + lane] : 0;
+      // while the MMAs run: this warp's part of C into L2 (lane: one row, two lines)
+      if (i < m) {
+        if (col0 < ncols) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + i * ldc + col0));
+        if (col0 + 16 < ncols) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + i * ldc + col0 + 16));
+      }
+      if (!mbar_wait(acc_full, (uint32_t)done & 1u) || *fail) {
+        *fail = 1;
+        break;
+      }
+      ++done;
+      tc_fence_after();
+      int64_t v[32];
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const uint32_t addr = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(cols0 + 16 * g);
+        // two neighbouring levels fit 32 bits: |I_l| < 2^23.4, so |128 I_l + I_(l+1)| < 2^31
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           uint32_t r[4][16];
 #pragma unroll
-          for (int l4 = 0; l4 < 4; ++l4)
-            tmem_ld_16cols_nowait(lane_addr + (uint32_t)(kOzN * (4 * half + l4) + 16 * g), r[l4]);
+          for (int l = 0; l < 4; ++l) tmem_ld_16cols_nowait(addr + (uint32_t)(kOzN * (4 * half + l)), r[l]);
           tmem_wait_ld();
-#define QGX_OZ_LEVEL(L)                                                                   \
-  _Pragma("unroll") for (int j = 0; j < 16; ++j) {                                        \
-    const long long tv = level_term<L>(__float2int_rn(__uint_as_float(r[(L) & 3][j])));  \
-    v[j] = (L) == 0 ? tv : v[j] + tv;                                                     \
-  }
-          if (half == 0) {
-            QGX_OZ_LEVEL(0)
-            QGX_OZ_LEVEL(1)
-            QGX_OZ_LEVEL(2)
-            QGX_OZ_LEVEL(3)
-          } else {
-            QGX_OZ_LEVEL(4)
-            QGX_OZ_LEVEL(5)
-            QGX_OZ_LEVEL(6)
-            QGX_OZ_LEVEL(7)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            auto level = [&](int l) { return __float2int_rn(__uint_as_float(r[l][j])); };
+            const int hi = 128 * level(0) + level(1), lo = 128 * level(2) + level(3);
+            // V = sum_l I_l 2^(38 - 7 l), levels 6 and 7 rounded to 2^-38 together
+            if (half == 0)
+              v[16 * g + j] = ((int64_t)hi << 31) + ((int64_t)lo << 17);
+            else
+              v[16 * g + j] += ((int64_t)hi << 3) + ((lo + 1024) >> 11);
           }
-#undef QGX_OZ_LEVEL
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty)) : "memory");
+      // C[i][j] -= 2^(e_i + e_j - 52) V_ij, eight columns a turn: lane = row into the buffer, then
+      // four rows of 64 bytes per access
+      const int rr = lane >> 3, cc = lane & 7;
+#pragma unroll
+      for (int c = 0; c < 32; c += kOzTurn) {
+#pragma unroll
+        for (int j = 0; j < kOzTurn; ++j)
+          tr[lane * kOzTurnLd + j] = fx_to_double(v[c + j], ei + __shfl_sync(0xffffffffu, ej, c + j) - 52);
+        __syncwarp();
+        double cv[8];
+        const int64_t j = col0 + c + cc;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int64_t r = row0 + 4 * k + rr;
+          cv[k] = r < m && j < ncols && j <= r ? C[r * ldc + j] : 0.0;
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) dt[rl * kOzDLd + 16 * g + j] = (double)v[j];
+        for (int k = 0; k < 8; ++k) {
+          const int64_t r = row0 + 4 * k + rr;
+          if (r < m && j < ncols && j <= r) C[r * ldc + j] = cv[k] - tr[(4 * k + rr) * kOzTurnLd + cc];
+        }
+        __syncwarp();
       }
     }
   }
   tc_fence_before();
-  __syncthreads();  // deltas complete; every role has left its loop
-  if (*fail) {
-    if (threadIdx.x == 0 && status) atomicExch(status, QGX_ERR_TIMEOUT);
-  } else {
-    // C[i][j] -= 2^(e_i + e_j - 52) V_ij on or below the diagonal, by all six warps (the
-    // producer and MMA warps are idle by now): warp w takes rows w, w + 6, ..., eight rows at a
-    // time with all their loads of C issued before the first update, so the loads' latencies
-    // overlap (lane l holds column l of each row)
-    constexpr int kBatch = 8, kRmwWarps = kOzThreads / 32;
-    int ej[kOzN / 32];
-    bool jin[kOzN / 32];
-#pragma unroll
-    for (int h = 0; h < kOzN / 32; ++h) {
-      const int64_t j = col0 + 32 * h + lane;
-      jin[h] = j < ncols;
-      ej[h] = jin[h] ? ex[b0 + j] : 0;
-    }
-#pragma unroll 1
-    for (int rb = warp; rb < kOzM; rb += kRmwWarps * kBatch) {
-      double cv[kBatch][kOzN / 32];
-      bool ok[kBatch][kOzN / 32];
-#pragma unroll
-      for (int r = 0; r < kBatch; ++r) {
-        const int rr = rb + kRmwWarps * r;  // a row of this tile (rr < kOzM) and of the matrix
-        const int64_t i = row0 + rr;
-#pragma unroll
-        for (int h = 0; h < kOzN / 32; ++h) {
-          const int64_t j = col0 + 32 * h + lane;
-          ok[r][h] = rr < kOzM && i < m && jin[h] && b0 + j <= a0 + i;
-          cv[r][h] = ok[r][h] ? C[i * ldc + j] : 0.0;
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < kBatch; ++r) {
-        const int rr = rb + kRmwWarps * r;
-        const int64_t i = row0 + rr;
-        const int ei = rr < kOzM && i < m ? ex[a0 + i] : 0;
-#pragma unroll
-        for (int h = 0; h < kOzN / 32; ++h) {
-          if (!ok[r][h]) continue;
-          const int cl = 32 * h + lane;
-          C[i * ldc + col0 + cl] = fma(-dt[rr * kOzDLd + cl], pow2(ei + ej[h] - 52), cv[r][h]);
-        }
-      }
-    }
-  }
-  if (*fail && warp == 4 && lane == 0) {
-    // no copy may land in shared memory after the CTA has left: wait (bounded) for the loads
-    // of the last stages issued
-    for (int kb = std::max(0, issued - kOzStages); kb < issued; ++kb)
-      mbar_wait(&full[kb % kOzStages], (uint32_t)((kb / kOzStages) & 1));
-  }
   __syncthreads();
+  if (*fail && threadIdx.x == 0 && status) atomicExch(status, QGX_ERR_TIMEOUT);
   if (warp == 0) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kOzTmemCols) : "memory");
   }
 }
 
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_fn() {
-  static std::once_flag once;
-  static EncodeTiled fn = nullptr;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiled>(p);
-  });
-  return fn;
-}
-
-// slices S[8][m][K] as a 3D tensor (K, m, 8); box 32 x box_rows x 8, 64-byte swizzle, rows past
-// m read as zeros
-int encode_slices(CUtensorMap* map, const __nv_bfloat16* S, int64_t m, int K, int box_rows) {
-  EncodeTiled enc = encode_fn();
-  if (!enc) return QGX_ERR_UNSUPPORTED;
-  const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)m, (cuuint64_t)kSlices};
-  const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)(m * K * 2)};
-  const cuuint32_t box[3] = {(cuuint32_t)kOzKB, (cuuint32_t)box_rows, (cuuint32_t)kSlices};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult cr = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(S), dims, strides, box,
-                          estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return cr == CUDA_SUCCESS ? QGX_OK : QGX_ERR_UNSUPPORTED;
-}
-
 struct CholWs {
-  __nv_bfloat16* s_panel[2];  // 8 x n x 256 digits of a trailing panel (two panels in flight)
+  uint8_t* s_panel[2];        // digits of a trailing panel's 256 columns (two panels in flight)
   int* e_panel[2];            // n row exponents each
-  __nv_bfloat16* s_block;     // 8 x n x 64 digits of the columns below a diagonal block
+  uint8_t* s_block;           // digits of the 64 columns below a diagonal block
   int* e_block;               // n row exponents
   BlockFactor* factor;        // the current diagonal block's
   RowBound bound;             // n row bounds
@@ -804,17 +784,18 @@ int64_t chol_layout(int64_t n, void* base, CholWs* ws) {
     off += al256(b);
     return o;
   };
-  const int64_t o_sp0 = take(kSlices * n * kPanel * 2), o_sp1 = take(kSlices * n * kPanel * 2);
+  const int64_t nr = slice_rows(n);
+  const int64_t o_sp0 = take(kSlices * nr * kPanel * 2), o_sp1 = take(kSlices * nr * kPanel * 2);
   const int64_t o_ep0 = take(n * 4), o_ep1 = take(n * 4);
-  const int64_t o_sb = take(kSlices * n * kBlk * 2), o_eb = take(n * 4), o_bf = take(sizeof(BlockFactor));
+  const int64_t o_sb = take(kSlices * nr * kBlk * 2), o_eb = take(n * 4), o_bf = take(sizeof(BlockFactor));
   const int64_t o_rf = take(n * 4), o_re = take(n * 4);
   if (base && ws) {
     char* b = static_cast<char*>(base);
-    ws->s_panel[0] = reinterpret_cast<__nv_bfloat16*>(b + o_sp0);
-    ws->s_panel[1] = reinterpret_cast<__nv_bfloat16*>(b + o_sp1);
+    ws->s_panel[0] = reinterpret_cast<uint8_t*>(b + o_sp0);
+    ws->s_panel[1] = reinterpret_cast<uint8_t*>(b + o_sp1);
     ws->e_panel[0] = reinterpret_cast<int*>(b + o_ep0);
     ws->e_panel[1] = reinterpret_cast<int*>(b + o_ep1);
-    ws->s_block = reinterpret_cast<__nv_bfloat16*>(b + o_sb);
+    ws->s_block = reinterpret_cast<uint8_t*>(b + o_sb);
     ws->e_block = reinterpret_cast<int*>(b + o_eb);
     ws->factor = reinterpret_cast<BlockFactor*>(b + o_bf);
     ws->bound.f = reinterpret_cast<float*>(b + o_rf);
@@ -823,22 +804,25 @@ int64_t chol_layout(int64_t n, void* base, CholWs* ws) {
   return off;
 }
 
-// C -= P P^T over the region of rows [r0, r0 + m) x columns [q0, q0 + ncols) of A, P the panel
-// sliced into S (ms rows, slice row r = matrix row s0 + r)
-int ozaki_region(double* A, int64_t lda, const __nv_bfloat16* S, const int* ex, int64_t ms, int64_t s0, int K,
-                 int64_t r0, int64_t m, int64_t q0, int64_t ncols, int32_t* status, cudaStream_t st,
-                 int64_t* kernels) {
+// C -= P P^T on and below the diagonal of the region of rows [r0, r0 + m) x columns
+// [r0, r0 + ncols) of A, P the K-column panel sliced into S (slice row r = matrix row s0 + r)
+int ozaki_region(double* A, int64_t lda, const uint8_t* S, const int* ex, int64_t s0, int K, int64_t r0, int64_t m,
+                 int64_t ncols, int32_t* status, cudaStream_t st, int64_t* kernels) {
   if (m <= 0 || ncols <= 0) return QGX_OK;
-  if (ms > 0x7fffffffLL || (m + kOzM - 1) / kOzM > 0x7fffffffLL || (ncols + kOzN - 1) / kOzN > 65535)
-    return QGX_ERR_UNSUPPORTED;
-  CUtensorMap ma, mb;
-  int rc = encode_slices(&ma, S, ms, K, kOzM);
-  if (rc == QGX_OK) rc = encode_slices(&mb, S, ms, K, kOzN);
-  if (rc != QGX_OK) return rc;
+  int64_t tiles = 0;  // as oz_tile enumerates them
+  const int64_t nr = (m + kOzM - 1) / kOzM, nc = (ncols + kOzN - 1) / kOzN;
+  for (int64_t g = 0; g * kOzGroup < nr; ++g) {
+    const int64_t rows = std::min<int64_t>(kOzGroup, nr - g * kOzGroup);
+    tiles += rows * std::min<int64_t>(nc, 2 * (g * kOzGroup + rows));
+  }
+  // several tiles per CTA hide the next tile's first loads behind the epilogue; fewer where the
+  // tiles would not fill the SMs four times over
+  const int64_t sms = device_sm_count();
+  const int per_cta = tiles >= 16 * sms ? 4 : tiles >= 4 * sms ? 2 : 1;
+  if (m > 0x7fffffffLL || tiles > 0x7fffffffLL) return QGX_ERR_UNSUPPORTED;
   QGX_CHECK_CUDA(cudaFuncSetAttribute(ozaki_syrk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzSmem));
-  const dim3 grid((unsigned)((m + kOzM - 1) / kOzM), (unsigned)((ncols + kOzN - 1) / kOzN));
-  ozaki_syrk_kernel<<<grid, kOzThreads, kOzSmem, st>>>(ma, mb, ex, m, ncols, (int)(r0 - s0), (int)(q0 - s0),
-                                                      K / kOzKB, A + r0 * lda + q0, lda, status);
+  ozaki_syrk_kernel<<<(unsigned)((tiles + per_cta - 1) / per_cta), kOzThreads, kOzSmem, st>>>(
+      S, ex, K / kOzKB, (int)(r0 - s0), m, ncols, A + r0 * lda + r0, lda, tiles, per_cta, status);
   ++*kernels;
   return launch_status();
 }
@@ -923,8 +907,8 @@ int chol_f64(double* A, int64_t n, int64_t lda, int* info, int32_t* status, void
       ++*kernels;
       if ((rc = launch_status()) != QGX_OK) return rc;
       // the block's columns update the rest of the panel (K = 64)
-      if (rb < pe && (rc = ozaki_region(A, lda, ws.s_block, ws.e_block, n - rb, rb, kBlk, rb, n - rb, rb, pe - rb,
-                                        status, aux, kernels)) != QGX_OK)
+      if (rb < pe && (rc = ozaki_region(A, lda, ws.s_block, ws.e_block, rb, kBlk, rb, n - rb, pe - rb, status, aux,
+                                        kernels)) != QGX_OK)
         return rc;
     }
     if (pe >= n) break;
@@ -938,14 +922,14 @@ int chol_f64(double* A, int64_t n, int64_t lda, int* info, int32_t* status, void
     // the strip updates the next panel's columns, which the previous panel's rest update (on st)
     // also updates: both read-modify-write the same entries, so the strip waits for it
     if (k >= 1) QGX_CHECK_CUDA(cudaStreamWaitEvent(aux, la->rest_done[(k - 1) & 1], 0));
-    if ((rc = ozaki_region(A, lda, ws.s_panel[b], ws.e_panel[b], ms, pe, kPanel, pe, ms, pe, pe2 - pe, status, aux,
+    if ((rc = ozaki_region(A, lda, ws.s_panel[b], ws.e_panel[b], pe, kPanel, pe, ms, pe2 - pe, status, aux,
                            kernels)) != QGX_OK)
       return rc;
     if (pe2 < n) {
       QGX_CHECK_CUDA(cudaEventRecord(la->strip_done[b], aux));
       QGX_CHECK_CUDA(cudaStreamWaitEvent(st, la->strip_done[b], 0));
-      if ((rc = ozaki_region(A, lda, ws.s_panel[b], ws.e_panel[b], ms, pe, kPanel, pe2, n - pe2, pe2, n - pe2, status,
-                             st, kernels)) != QGX_OK)
+      if ((rc = ozaki_region(A, lda, ws.s_panel[b], ws.e_panel[b], pe, kPanel, pe2, n - pe2, n - pe2, status, st,
+                             kernels)) != QGX_OK)
         return rc;
       QGX_CHECK_CUDA(cudaEventRecord(la->rest_done[b], st));
     }
