@@ -121,21 +121,37 @@ constexpr float kFxHigh = 4.656612873077393e-10f;  // 2^-31: the unit of Fx::h
 // update of its later columns, the next owner first of all. A dead group costs nothing, so the
 // executed multiply-adds are those of the triangle.
 
-// s[e] -= sum over the four columns k of x_k y_k[e], e the four columns of the warp's group;
-// x: entry of the lane's row in column k (stride ldx), y: the group's rows of column k
+// A group of four columns as an update takes it: x, the entries of the lane's row (negated), and
+// y, the rows of the columns that are updated
+struct GroupUpdate {
+  Fx x[4], y[4][4];
+  // x: entry of the lane's row in the group's first column (stride ldx); y: the updated group's
+  // first row of it (stride ldy)
+  __device__ inline GroupUpdate(const Fx* __restrict__ xp, int ldx, const Fx* __restrict__ yp, int ldy) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      x[k] = xp[k * ldx];
+      x[k].h = -x[k].h;
+      x[k].l = -x[k].l;
+      const int4 a = *reinterpret_cast<const int4*>(yp + k * ldy), b = *reinterpret_cast<const int4*>(yp + k * ldy + 2);
+      y[k][0] = Fx{a.x, a.y};
+      y[k][1] = Fx{a.z, a.w};
+      y[k][2] = Fx{b.x, b.y};
+      y[k][3] = Fx{b.z, b.w};
+    }
+  }
+  __device__ inline void column(int e, int64_t* s1, int64_t* s2) const {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) fx_mad(s1[e], s2[e], x[k], y[k][e]);
+  }
+};
+
+// s[e] -= sum over the group's columns k of x_k y_k[e], e the four columns of the warp's group
 __device__ inline void apply_group(const Fx* __restrict__ x, int ldx, const Fx* __restrict__ y, int ldy, int64_t* s1,
                                    int64_t* s2) {
+  const GroupUpdate u(x, ldx, y, ldy);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    Fx v = x[k * ldx];
-    v.h = -v.h;
-    v.l = -v.l;
-    const int4 a = *reinterpret_cast<const int4*>(y + k * ldy), b = *reinterpret_cast<const int4*>(y + k * ldy + 2);
-    fx_mad(s1[0], s2[0], v, Fx{a.x, a.y});
-    fx_mad(s1[1], s2[1], v, Fx{a.z, a.w});
-    fx_mad(s1[2], s2[2], v, Fx{b.x, b.y});
-    fx_mad(s1[3], s2[3], v, Fx{b.z, b.w});
-  }
+  for (int e = 0; e < 4; ++e) u.column(e, s1, s2);
 }
 
 constexpr int kPotrfThreads = 512;
@@ -153,44 +169,57 @@ struct PotrfShared {
   int kfail;             // first column whose pivot failed
 };
 
-// the warp's 32 rows (from row0) of the columns k0 .. k0 + 3, all updates taken: scaled and
-// published. PIVOT: the columns' pivots are among these rows and are inverted here (by every
-// lane alike); else they were, a barrier ago.
+// the warp's 32 rows (from row0) of the columns k0 .. k0 + 3, scaled and published; all updates are
+// taken but the previous group's, which is taken here (its share of column k0 first: the chain
+// waits for nothing else). PIVOT: the columns' pivots are among these rows and are inverted here
+// (by every lane alike); else they were, a barrier ago.
 template <bool PIVOT>
 __device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, int64_t* s1, int64_t* s2) {
   const int i = row0 + lane;
   float squares = sh.squares[i];
   bool bad = sh.bad[i] != 0;
   int kfail = sh.kfail;
+  // the first group has no previous one: any finite operand times zero
+  GroupUpdate prev(&sh.l[k0 > 0 ? k0 - 4 : 0][i], kPotrfLd, &sh.l[k0 > 0 ? k0 - 4 : 0][k0], kPotrfLd);
+  if (k0 == 0) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) prev.x[k] = Fx{0, 0};
+  }
+  prev.column(0, s1, s2);
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    const int k = k0 + e;
-    FxPivot piv;
+    const int k = k0 + e, src = k - row0;
+    Fx x;
+    bool in_range, positive;
     if (PIVOT) {
-      const int src = k - row0;
-      const bool fail = kfail < kBlk || __shfl_sync(0xffffffffu, (int)bad, src) != 0;
-      const int64_t p1 = __shfl_sync(0xffffffffu, s1[e], src), p2 = __shfl_sync(0xffffffffu, s2[e], src);
-      uint64_t u;
-      piv = fx_rsqrt(fail ? -1 : p1, fail ? 0 : p2, &u);
-      if (piv.m == 0) kfail = min(kfail, k);
+      const int64_t p1 = __shfl_sync(0xffffffffu, bad ? 0 : s1[e], src), p2 = __shfl_sync(0xffffffffu, s2[e], src);
+      const FxInverse inv = fx_inverse(kfail < kBlk ? 0 : p1, p2);
+      positive = inv.Y != 0;
+      in_range = fx_in_range(s1[e], inv.t);
+      x = fx_split(fx_scale(s1[e], s2[e], inv, in_range));
+      if (!positive) kfail = min(kfail, k);
       if (lane == 0) {
-        sh.piv[k] = piv;
-        sh.u[k] = u;
+        sh.piv[k] = fx_pivot(inv);
+        sh.u[k] = inv.u;
       }
     } else {
-      piv = sh.piv[k];
+      const FxPivot piv = sh.piv[k];
+      positive = piv.m != 0;
+      in_range = fx_in_range(s1[e], piv.t);
+      x = fx_split(fx_scale(s1[e], s2[e], piv, in_range));
     }
-    bool ok;
-    Fx x = fx_split(fx_scale(s1[e], s2[e], piv, &ok));
+    if (e == 0) {
+#pragma unroll
+      for (int f = 1; f < 4; ++f) prev.column(f, s1, s2);
+    }
     const float xv = (float)x.h * kFxHigh;
     const float sq = fmaf(xv, xv, squares);
-    const bool below = i > k && piv.m != 0;
-    bad |= below && (!ok || sq > kFullRow);
+    const bool below = i > k && positive;
+    bad |= below && (!in_range || sq > kFullRow);
     if (below && !bad)
       squares = sq;
     else
       x = Fx{0, 0};
-    sh.l[k][i] = x;
     Fx y[4];
 #pragma unroll
     for (int f = e + 1; f < 4; ++f) {
@@ -201,6 +230,7 @@ __device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, 
         y[f] = sh.l[k][k0 + f];
       }
     }
+    sh.l[k][i] = x;
     x.h = -x.h;
     x.l = -x.l;
 #pragma unroll
@@ -217,9 +247,9 @@ __device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, 
 // hold rows 0 .. 31, one column group each, and eight rows 32 .. 63, two groups each; the lower
 // rows follow the upper ones by one group. The chain of 64 pivots bounds the kernel (one CTA), so
 // the lower rows' multiply-adds and the stores are kept off the sub-cores that the chain runs on.
-// Measured: 34 us a block (62 us in FP64; of a column's 850 clocks the inverse square root takes
-// 330 and the scaling 140). The factorisation with this kernel and the next: 1.04 ms at n = 1024
-// (1.60 in FP64), 4.6 at 4096 (7.4), 14.0 at 8192 (20.4), 618 at 32768 (668).
+// Measured: 30 us a block (62 us in FP64), about 780 clocks a column, of which the inverse square
+// root and the scaling take 500. With this kernel and the next the factorisation takes 0.99 ms at
+// n = 1024 (1.60 with FP64 blocks) and 4.4 at 4096 (7.4).
 __global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
                                                                     int nb, RowBound bound,
                                                                     BlockFactor* __restrict__ out,
@@ -278,14 +308,13 @@ __global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __re
     const int g = lower ? step - 1 : step;  // the group these rows solve
     if (g >= 0 && g < 8) {
       const int k0 = 4 * (g - 1);  // the previous group's first column
-      if (g0 >= g) {
-        if (g > 0) apply_group(&sh.l[k0][i], kPotrfLd, &sh.l[k0][4 * g0], kPotrfLd, s1, s2);
-        if (g0 == g) {
-          if (lower)
-            solve_group<false>(sh, 4 * g, row0, lane, s1, s2);
-          else
-            solve_group<true>(sh, 4 * g, row0, lane, s1, s2);
-        }
+      if (g0 == g) {
+        if (lower)
+          solve_group<false>(sh, 4 * g, row0, lane, s1, s2);
+        else
+          solve_group<true>(sh, 4 * g, row0, lane, s1, s2);
+      } else if (g0 > g && g > 0) {
+        apply_group(&sh.l[k0][i], kPotrfLd, &sh.l[k0][4 * g0], kPotrfLd, s1, s2);
       }
       if (lower && g > 0) apply_group(&sh.l[k0][i], kPotrfLd, &sh.l[k0][32 + 4 * g0], kPotrfLd, s1 + 4, s2 + 4);
     }
@@ -295,10 +324,10 @@ __global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __re
   for (int g = 8; g < 16; ++g) {
     const int k0 = 4 * (g - 1);
     if (lower) {
-      if (g0 >= g - 8) {
+      if (g0 == g - 8)
+        solve_group<true>(sh, 4 * g, row0, lane, s1 + 4, s2 + 4);
+      else if (g0 > g - 8)
         apply_group(&sh.l[k0][i], kPotrfLd, &sh.l[k0][32 + 4 * g0], kPotrfLd, s1 + 4, s2 + 4);
-        if (g0 == g - 8) solve_group<true>(sh, 4 * g, row0, lane, s1 + 4, s2 + 4);
-      }
     } else if (g0 == g - 8) {
       store_group(g0, 0);
     } else if (g0 == ((g - 7) & 7)) {
@@ -357,11 +386,12 @@ __device__ inline void trsm_group(TrsmShared& sh, int k0, int lane, int64_t* s1,
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int k = k0 + e;
-    bool ok;
-    Fx x = fx_split(fx_scale(s1[e], s2[e], sh.f.piv[k], &ok));
+    const FxPivot piv = sh.f.piv[k];
+    const bool in_range = fx_in_range(s1[e], piv.t);
+    Fx x = fx_split(fx_scale(s1[e], s2[e], piv, in_range));
     const float xv = (float)x.h * kFxHigh;
     squares = fmaf(xv, xv, squares);
-    bad |= !ok || squares > kFullRow;
+    bad |= !in_range || squares > kFullRow;
     if (bad) x = Fx{0, 0};
     sh.x[k][lane] = x;
     x.h = -x.h;

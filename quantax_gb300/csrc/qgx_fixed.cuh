@@ -107,11 +107,10 @@ __host__ __device__ inline void fx_mad(int64_t& s1, int64_t& s2, const Fx& nx, c
   mad_wide(s2, nx.l, y.h);
 }
 
-// (s1 2^-62 + s2 2^-91) 2^t in units of 2^-62; modulo 2^64, exact whenever the result fits
+// (s1 2^-62 + s2 2^-91) 2^t in units of 2^-62, 0 <= t <= 29; modulo 2^64, exact whenever the
+// result fits
 __host__ __device__ inline int64_t fx_combine(int64_t s1, int64_t s2, int t) {
-  const uint64_t a = (uint64_t)s1 << t;
-  const uint64_t b = t <= 29 ? (uint64_t)(s2 >> (29 - t)) : (uint64_t)s2 << (t - 29);
-  return (int64_t)(a + b);
+  return (int64_t)(((uint64_t)s1 << t) + (uint64_t)(s2 >> (29 - t)));
 }
 
 // floor of a b / 2^64 up to 2 units below, a < 3/4 2^64 or b < 2^63, the other below 2^63
@@ -130,58 +129,80 @@ __host__ __device__ inline Fx fx_split(int64_t X) {
 }
 __host__ __device__ inline int64_t fx_join(const Fx& x) { return ((int64_t)x.h << 29) + x.l; }
 
-// Inverse square root of a pivot 0 < v <= 1/2: 1 / sqrt(v) = m 2^-62 2^t, m 2^-62 in (1, 2].
-// A float estimate y0 of the normalised pivot u in [1/4, 1) and one third-order step,
-// y = y0 (1 + h/2 + 3 h^2/8) with h = 1 - u y0^2 (|h| < 2^-20.5; error 5 h^3 / 16).
+// Inverse square root of a pivot v, 2^-58 <= v <= 1/2 (below that the pivot counts as not
+// positive: it is noise of its row): 1 / sqrt(v) = Y 2^-23 (1 + c 2^-60) 2^t from a float estimate
+// Y 2^-23 in [1, 2] for the normalised pivot u in [1/4, 1) and one third-order step
+// c = h/2 + 3 h^2/8 with h = 1 - u y0^2 (|h| < 2^-20.5; error 5 h^3 / 16).
+struct FxInverse {
+  uint32_t Y;  // 0: the pivot is not positive
+  int t;
+  int64_t c;
+  uint64_t u;  // units of 2^-62
+};
+__host__ __device__ inline FxInverse fx_inverse(int64_t s1, int64_t s2) {
+  const int64_t v0 = fx_combine(s1, s2, 0);
+  const bool pos = v0 >= 16;
+  const int t2 = (clz64((uint64_t)(pos ? v0 : 1LL << 60)) - 2) & ~1;
+  FxInverse r;
+  r.u = (uint64_t)(pos ? v0 : 1LL << 60) << t2;  // in [2^60, 2^62)
+  const float f = (float)(uint32_t)(r.u >> 32);  // 2^30 u; its inverse root's bits less those of
+  uint32_t Y;                                    // 2^-16 are y0 2^23
+#ifdef __CUDA_ARCH__
+  float y0;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(f));
+  Y = (uint32_t)__float_as_int(y0) - 0x37800000u;
+#else
+  const float y0 = 1.0f / std::sqrt(f);
+  memcpy(&Y, &y0, 4);
+  Y -= 0x37800000u;
+#endif
+  const int64_t h = (1LL << 60) - (int64_t)fx_mulhi(r.u << 1, ((uint64_t)Y * Y) << 15);  // 2^-60
+  const int hh = (int)(h >> 11);                                                         // 2^-49
+  r.c = (h >> 1) + (((int64_t)(3 * hh) * hh) >> 41);
+  r.Y = pos ? Y : 0;
+  r.t = t2 >> 1;
+  return r;
+}
+
+// the same as one factor: 1 / sqrt(v) = m 2^-62 2^t
 struct FxPivot {
   uint64_t m;  // 0: the pivot is not positive
   int t;
 };
-__host__ __device__ inline FxPivot fx_rsqrt(int64_t s1, int64_t s2, uint64_t* u_out) {
-  const int64_t v0 = fx_combine(s1, s2, 0);
-  const uint32_t vh = (uint32_t)((uint64_t)v0 >> 32);
-  // u = v 2^t2 in units of 2^-62, in [2^60, 2^62), t2 even
-  int t2;
-  if (vh >= 4) {  // the common case, with 32-bit shift counts throughout
-    t2 = (clz64((uint64_t)vh) - 34) & ~1;
-  } else {
-    t2 = (clz64((uint64_t)v0 | 1) - 2) & ~1;
-  }
-  const uint64_t u = (uint64_t)fx_combine(s1, s2, t2);
-  const float f = (float)(uint32_t)(u >> 32);  // 2^30 u
-#ifdef __CUDA_ARCH__
-  float y0;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(f));
-  const uint32_t Y = (uint32_t)__float_as_int(y0 * 32768.0f) - 0x3F000000u;
-#else
-  const float y0 = 32768.0f / std::sqrt(f);
-  uint32_t Y;
-  memcpy(&Y, &y0, 4);
-  Y -= 0x3F000000u;
-#endif
-  // y0 in [1, 2]: its bits less those of 0.5 are y0 2^23
-  const int64_t h = (1LL << 60) - (int64_t)fx_mulhi(u << 1, ((uint64_t)Y * Y) << 15);  // 2^-60
-  const int hh = (int)(h >> 9);                                                        // 2^-51
-  const int64_t h2 = ((int64_t)hh * hh) >> 42;                                         // 2^-60
-  const int64_t c = (h >> 1) + ((3 * h2) >> 3);
+__host__ __device__ inline FxPivot fx_pivot(const FxInverse& p) {
   FxPivot r;
-  r.m = v0 > 0 ? ((uint64_t)Y << 39) + (uint64_t)((c * (int64_t)Y) >> 21) : 0;
-  r.t = v0 > 0 ? t2 >> 1 : 0;
-  *u_out = u;
+  r.m = ((uint64_t)p.Y << 39) + (uint64_t)((p.c * (int64_t)p.Y) >> 21);
+  r.t = p.t;
   return r;
 }
 
 // sqrt(v) of the pivot in units of 2^-(61 + t)
 __host__ __device__ inline int64_t fx_sqrt(uint64_t u, const FxPivot& p) { return (int64_t)fx_mulhi(u << 1, p.m); }
 
-// x = v 2^t m 2^-62 in units of 2^-60; *ok = false when |v| 2^t is not below 3/4 (no row of a
-// positive definite matrix gets there: |x| <= sqrt(1/2) and m 2^-62 > 1)
-__host__ __device__ inline int64_t fx_scale(int64_t s1, int64_t s2, const FxPivot& piv, bool* ok) {
+// whether |v| 2^t is below 3/4: no row of a positive definite matrix exceeds it (|x| <= sqrt(1/2)
+// and the mantissa of 1 / sqrt(v) is at least 1)
+__host__ __device__ inline bool fx_in_range(int64_t s1, int t) {
   const int top = (int)(s1 >> 32);
-  *ok = (top < 0 ? -top : top) <= ((3 << 28) >> piv.t);
+  return (top < 0 ? -top : top) <= ((3 << 28) >> t);
+}
+
+// x = v 2^t m 2^-62 in units of 2^-60 (0 unless in range)
+__host__ __device__ inline int64_t fx_scale(int64_t s1, int64_t s2, const FxPivot& piv, bool in_range) {
   const int64_t w = fx_combine(s1, s2, piv.t);
-  const uint64_t a = *ok ? (w < 0 ? 0ULL - (uint64_t)w : (uint64_t)w) : 0;
-  const int64_t X = (int64_t)((fx_mulhi(a << 1, piv.m) + 2) >> 1);
+  const uint64_t a = in_range ? (w < 0 ? 0ULL - (uint64_t)w : (uint64_t)w) : 0;
+  const int64_t X = (int64_t)((fx_mulhi(a << 1, piv.m) + 1) >> 1);
+  return w < 0 ? -X : X;
+}
+
+// the same from the inverse's parts: v y0 does not wait for c, so the chain from a pivot to its
+// column is the shorter by one multiplication
+__host__ __device__ inline int64_t fx_scale(int64_t s1, int64_t s2, const FxInverse& inv, bool in_range) {
+  const int64_t w = fx_combine(s1, s2, inv.t);
+  const uint64_t a = in_range ? (w < 0 ? 0ULL - (uint64_t)w : (uint64_t)w) : 0;
+  const uint64_t T = fx_mulhi(a << 1, (uint64_t)inv.Y << 39);  // 2^-61, below 2^62
+  const uint64_t c = (uint64_t)(inv.c < 0 ? -inv.c : inv.c) << 23;  // 2^-83, below 2^63
+  const uint64_t d = fx_mulhi(T << 1, c) >> 20;  // (2^-62 2^-83 2^64) 2^20: 2^-61
+  const int64_t X = (int64_t)((inv.c < 0 ? T - d : T + d) + 1) >> 1;
   return w < 0 ? -X : X;
 }
 
