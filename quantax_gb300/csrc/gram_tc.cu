@@ -6,8 +6,8 @@
 //                    column block, 128B-swizzled, into a ring of kStages shared-memory stages;
 //   warp 5 / lane 0  MMA issuer: tcgen05.mma M=128 N=128 (K = 8 for tf32, 16 for bf16; four
 //                    per 128-byte k-block); tcgen05.commit frees a stage when its MMAs are done;
-//   warps 6-9        (split tf32 only) write the low parts lo = x - tf32(x) of the staged
-//                    operands beside them;
+//   warps 6-9        (split tf32 only) move A's high and low parts to tensor memory and write
+//                    the low parts lo = x - tf32(x) of B beside it;
 //   warps 0-3        epilogue (warp w owns TMEM lanes 32w..32w+31, i.e. tile rows).
 // K is accumulated in chunks of kChunkElems elements, alternately in two 128-column TMEM
 // accumulators, each chunk starting from zero. The epilogue adds every finished chunk into
@@ -38,14 +38,21 @@ constexpr int kBlockBytes = kTile * kRowBytes;  // one operand block of a stage
 constexpr int kChunkElems = 256;  // K elements accumulated in TMEM before the epilogue takes them
 template <int KIND>
 struct GramCfg {
-  static constexpr int kStageBytes = (KIND == 2 ? 4 : 2) * kBlockBytes;  // A, B (+ A lo, B lo)
-  static constexpr int kStages = 3;
+  // A and B (and, split tf32, the low parts of B); as many stages as shared memory holds: a stage
+  // is occupied from the start of its load to the end of its MMAs, far longer than those take
+  // (six stages instead of three: TF32 95.3 -> 88.2 ms, BF16 48.4 -> 47.7 ms at 32768 x 34944)
+  static constexpr int kStageBytes = (KIND == 2 ? 3 : 2) * kBlockBytes;
+  static constexpr int kStages = KIND == 2 ? 4 : 6;
   static constexpr int kThreads = KIND == 2 ? 320 : 192;  // epilogue 0-3, producer 4, MMA 5, split 6-9
   static constexpr size_t kSmem = 1024 + (size_t)kStages * kStageBytes + 256;
   static constexpr int kElems = KIND == 1 ? 64 : 32;      // elements per 128-byte k-block
   static constexpr int kChunkBlocks = kChunkElems / kElems;
 };
-constexpr uint32_t kTmemCols = 256;  // two chunk accumulators
+constexpr uint32_t kAccCols = 256;  // two chunk accumulators
+// split tf32: beside them the A operands of the four stages, 32 columns of high and 32 of low parts
+template <int KIND>
+constexpr uint32_t tmem_cols() { return KIND == 2 ? 512 : kAccCols; }
+__device__ inline uint32_t tmem_a(uint32_t tmem, int stage) { return tmem + kAccCols + 64u * (uint32_t)stage; }
 
 // K-major operand tile, 128-byte rows, 128B swizzle: 8-row core groups 1024 bytes apart
 __device__ inline uint64_t smem_desc_sw128(uint32_t saddr) {
@@ -81,6 +88,29 @@ __device__ inline void mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t acc
   }
 }
 
+// the same (TF32) with A in tensor memory
+__device__ inline void mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(b), "r"(instr_desc<2>()), "r"(accumulate));
+}
+
+// 32 columns of this warp's 32 TMEM lanes from registers (tcgen05.wait::st completes them)
+__device__ inline void tmem_st_32cols(uint32_t taddr, const float (&v)[32]) {
+  uint32_t r[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(v[i]);
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+      "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};" ::"r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+      "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
+      "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
+      : "memory");
+}
+
 // the TF32 value the tensor core takes from an FP32 operand: the 10 leading explicit mantissa
 // bits, the 13 below them ignored
 __device__ inline float tf32_hi(float x) { return __uint_as_float(__float_as_uint(x) & 0xFFFFE000u); }
@@ -100,7 +130,7 @@ __global__ void __launch_bounds__(GramCfg<KIND>::kThreads, 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
   uint64_t* empty = full + kStages;
-  uint64_t* split = empty + kStages;  // KIND 2: operands split into hi / lo
+  uint64_t* split = empty + kStages;      // KIND 2: A in tensor memory, low parts of B written
   uint64_t* acc_full = split + kStages;   // two: a chunk accumulator is complete
   uint64_t* acc_empty = acc_full + 2;     // two: the epilogue has taken a chunk accumulator
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
@@ -135,7 +165,7 @@ __global__ void __launch_bounds__(GramCfg<KIND>::kThreads, 1)
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(kTmemCols)
+                 "r"(tmem_cols<KIND>())
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -183,44 +213,68 @@ __global__ void __launch_bounds__(GramCfg<KIND>::kThreads, 1)
         }
         tc_fence_after();
         const uint32_t base = smem_u32(smem + s * kStageBytes);
-        const uint64_t da = smem_desc_sw128(base);
         const uint64_t db = smem_desc_sw128(base + kBlockBytes);
+        if constexpr (KIND == 2) {
+          const uint32_t ta = tmem_a(tmem, s);
+          const uint64_t lb = smem_desc_sw128(base + 2 * kBlockBytes);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)  // 32 bytes of K per instruction
-          mma<KIND>(acc, da + 2 * kk, db + 2 * kk, (first && kk == 0) ? 0u : 1u);
-        if (KIND == 2) {
-          const uint64_t la = smem_desc_sw128(base + 2 * kBlockBytes);
-          const uint64_t lb = smem_desc_sw128(base + 3 * kBlockBytes);
+          for (int kk = 0; kk < 4; ++kk)  // 32 bytes of K per instruction
+            mma_ta(acc, ta + 8 * kk, db + 2 * kk, (first && kk == 0) ? 0u : 1u);
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
-            mma<KIND>(acc, da + 2 * kk, lb + 2 * kk, 1u);
-            mma<KIND>(acc, la + 2 * kk, db + 2 * kk, 1u);
+            mma_ta(acc, ta + 8 * kk, lb + 2 * kk, 1u);
+            mma_ta(acc, ta + 32 + 8 * kk, db + 2 * kk, 1u);
           }
+        } else {
+          const uint64_t da = smem_desc_sw128(base);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma<KIND>(acc, da + 2 * kk, db + 2 * kk, (first && kk == 0) ? 0u : 1u);
         }
         mma_commit(&empty[s]);
         if (last) mma_commit(&acc_full[c & 1]);
       }
     }
   } else if (KIND == 2 && warp >= 6) {
-    // split x = hi + lo: the tensor core reads an FP32 operand as TF32 by ignoring its 13
-    // low mantissa bits, so the staged x itself is hi; lo = x - hi is exact and goes to a
-    // second buffer in the same swizzled layout (the tensor core reads lo truncated too)
-    const int t = threadIdx.x - 192;
+    // split x = hi + lo, hi the TF32 value the tensor core takes from x, lo = x - hi exact. A's
+    // parts go to tensor memory (thread = row = lane), so that the twelve MMAs of a k-block read
+    // only B from shared memory: staged A tiles and low parts were read twelve times over there,
+    // 250 bytes a clock with the loads and the split: 5.44 -> 4.93 ms at 8192 x 16640, 172.9 ->
+    // 161.7 at 32768 x 34944. (Without any split work it takes 4.46: the MMAs of N = 128 themselves,
+    // about 105 clocks each, bound it now.) B's staged words are its high parts as they are (the tensor core ignores the 13 low mantissa bits); its low parts
+    // are written beside them in the same swizzled layout
+    const int t = threadIdx.x - 192, q = warp & 3, row = 32 * q + lane;
     for (int64_t kb = 0; kb < nkb && !*fail; ++kb) {
       const int s = (int)(kb % kStages);
-      const uint32_t ph = (uint32_t)((kb / kStages) & 1);
-      if (!mbar_wait(&full[s], ph)) {
+      if (!mbar_wait(&full[s], (uint32_t)((kb / kStages) & 1))) {
         *fail = 1;
         break;
       }
-      const float4* x = reinterpret_cast<const float4*>(smem + s * kStageBytes);
-      float4* lo = reinterpret_cast<float4*>(smem + s * kStageBytes + 2 * kBlockBytes);
-#pragma unroll 4
-      for (int e = t; e < 2 * kBlockBytes / 16; e += 128) {
-        const float4 v = x[e];
-        lo[e] = make_float4(v.x - tf32_hi(v.x), v.y - tf32_hi(v.y), v.z - tf32_hi(v.z), v.w - tf32_hi(v.w));
+      uint8_t* stage = smem + s * kStageBytes;
+      float hi[32], lo[32];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float4 v = *reinterpret_cast<const float4*>(stage + row * kRowBytes + ((c ^ (row & 7)) << 4));
+        const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          hi[4 * c + j] = tf32_hi(x[j]);
+          lo[4 * c + j] = x[j] - hi[4 * c + j];
+        }
       }
+      const uint32_t ta = tmem_a(tmem, s) + ((uint32_t)(32 * q) << 16);
+      tmem_st_32cols(ta, hi);
+      tmem_st_32cols(ta + 32, lo);
+      const float4* x = reinterpret_cast<const float4*>(stage + kBlockBytes);
+      float4* xl = reinterpret_cast<float4*>(stage + 2 * kBlockBytes);
+#pragma unroll
+      for (int e = 0; e < kBlockBytes / 16 / 128; ++e) {
+        const float4 v = x[t + 128 * e];
+        xl[t + 128 * e] = make_float4(v.x - tf32_hi(v.x), v.y - tf32_hi(v.y), v.z - tf32_hi(v.z), v.w - tf32_hi(v.w));
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tc_fence_before();
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&split[s])) : "memory");
     }
   }
@@ -281,7 +335,7 @@ __global__ void __launch_bounds__(GramCfg<KIND>::kThreads, 1)
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols<KIND>()) : "memory");
   }
 }
 
