@@ -694,154 +694,265 @@ __device__ inline float gelu_tanh_grad(float x) {
 
 constexpr int kJacThreads = 256;
 
-// dW[o][i][t] += sum_r g[k][o][r] in[i][nbr(r,t)] and db[o] = sum_r g[k][o][r] for both
-// cotangents k, written to the O rows at the layer's parameter offset (reference layout
-// (o, i, ky, kx) then bias). Thread = (cotangent, 4 output channels, input channel, half of
-// the sites); the two halves are summed with a lane shuffle.
+// ---- the passes of the Jacobian, one sample per CTA ----
+// Two threads per site (h = 0, 1) hold C / 2 channels each, in packed pairs; a warp's threads share
+// h, so weight loads are broadcasts. N sites rounded up to whole warps per h.
+
+// C / 2 weights (8-byte aligned, 16 where C / 2 is a multiple of 4) as pairs
 template <int C>
-__device__ inline void weight_grads(const float* __restrict__ g /*[2][C][N]*/, const float* __restrict__ in /*[cin][N]*/,
-                                    int cin, const int16_t* __restrict__ nbr, int N, bool has_bias,
-                                    float* __restrict__ o_re, float* __restrict__ o_im, bool accumulate) {
-  constexpr int G = C / 4;
-  const int items = 2 * G * cin * 2;  // cotangent x o-group x input channel x half
-  // every lane of a warp runs the same iterations (blockDim is a multiple of 32), so the
-  // full-warp shuffles below always see all 32 lanes; lanes past `items` add zeros
-  for (int base = 0; base < items; base += blockDim.x) {
-    const int it = base + threadIdx.x;
-    const bool active = it < items;
-    const int half = it & 1;
-    const int rest = active ? it >> 1 : 0;
-    const int i = rest % cin;
-    const int og = (rest / cin) % G;
-    const int k = rest / (cin * G);
-    float acc[4][9];
+__device__ inline void load_half(const float* __restrict__ w, float2 (&v)[C / 4]) {
+  if constexpr ((C / 2) % 4 == 0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int e = 0; e < C / 8; ++e) {
+      const float4 q = reinterpret_cast<const float4*>(w)[e];
+      v[2 * e] = make_float2(q.x, q.y);
+      v[2 * e + 1] = make_float2(q.z, q.w);
+    }
+  } else {
 #pragma unroll
-      for (int t = 0; t < 9; ++t) acc[q][t] = 0.0f;
-    float bacc[4] = {0.f, 0.f, 0.f, 0.f};
-    const float* gk = g + (int64_t)k * C * N + (4 * og) * N;
-    const float* ini = in + (int64_t)i * N;
-    const int r0 = half ? N / 2 : 0, r1 = !active ? 0 : (half ? N : N / 2);
-    for (int r = r0; r < r1; ++r) {
-      float gv[4];
+    for (int e = 0; e < C / 4; ++e) v[e] = reinterpret_cast<const float2*>(w)[e];
+  }
+}
+
+// emit(o, r, y): output channel o of site r is y = bias[o] + sum_{i,tap} W[i][tap][o] in[i][nbr(r,tap)]
+// (the forward's chain of operations)
+template <int C, class Emit>
+__device__ inline void conv_sites(const float* __restrict__ in, int cin, const float* __restrict__ w,
+                                  const int16_t* __restrict__ nbr, int N, Emit emit) {
+  constexpr int CO = C / 2;
+  const int per = (N + 31) & ~31;
+  for (int it = threadIdx.x; it < 2 * per; it += kJacThreads) {
+    const int h = it >= per, r = it - h * per;
+    if (r >= N) continue;
+    int nb[9];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) gv[q] = gk[q * N + r];
+    for (int t = 0; t < 9; ++t) nb[t] = nbr[r * 9 + t];
+    float2 acc[CO / 2];
+    load_half<C>(w + cin * 9 * C + h * CO, acc);
+#pragma unroll 2
+    for (int i = 0; i < cin; ++i) {
 #pragma unroll
       for (int t = 0; t < 9; ++t) {
-        const float v = ini[nbr[r * 9 + t]];
+        const float x = in[i * N + nb[t]];
+        float2 ww[CO / 2];
+        load_half<C>(w + (i * 9 + t) * C + h * CO, ww);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[q][t] = fmaf(gv[q], v, acc[q][t]);
+        for (int e = 0; e < CO / 2; ++e) fma_pair(acc[e], make_float2(x, x), ww[e]);
       }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) bacc[q] += gv[q];
     }
-    // the two halves sit in adjacent lanes (items are laid out half-fastest)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-#pragma unroll
-      for (int t = 0; t < 9; ++t) acc[q][t] += __shfl_xor_sync(0xffffffffu, acc[q][t], 1);
-      bacc[q] += __shfl_xor_sync(0xffffffffu, bacc[q], 1);
-    }
-    if (active && half == 0) {
-      float* row = k == 0 ? o_re : o_im;
-      if (row) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int o = 4 * og + q;
-#pragma unroll
-          for (int t = 0; t < 9; ++t) {
-            float* dst = row + ((int64_t)o * cin + i) * 9 + t;
-            *dst = accumulate ? *dst + acc[q][t] : acc[q][t];
-          }
-          if (has_bias && i == 0) {
-            float* dst = row + (int64_t)C * cin * 9 + o;
-            *dst = accumulate ? *dst + bacc[q] : bacc[q];
-          }
-        }
-      }
+    for (int e = 0; e < CO / 2; ++e) {
+      emit(h * CO + 2 * e, r, acc[e].x);
+      emit(h * CO + 2 * e + 1, r, acc[e].y);
     }
   }
 }
 
-// gin[k][i][r] = sum_{t,o} W[o][i][t] g[k][o][nbr(r, 8 - t)] (transposed convolution), WT = W as [t][o][i]
-template <int C>
-__device__ inline void input_grads(const float* __restrict__ g, const float* __restrict__ WT, int cin,
-                                   const int16_t* __restrict__ nbr, int N, float* __restrict__ gin) {
-  for (int it = threadIdx.x; it < 2 * N; it += blockDim.x) {
-    const int k = it / N, r = it - k * N;
-    float acc[C];
+// emit(i, r, v): v[k] = sum_{t,o} W[o][i][t] g[k][o][nbr(r, 8 - t)] (transposed convolution), WT = W
+// as [t][o][i]; the NK cotangents share the weight loads
+template <int C, int NK, class Emit>
+__device__ inline void input_grads(const float* __restrict__ g, const float* __restrict__ WT,
+                                   const int16_t* __restrict__ nbr, int N, Emit emit) {
+  constexpr int CO = C / 2;
+  const int per = (N + 31) & ~31;
+  for (int it = threadIdx.x; it < 2 * per; it += kJacThreads) {
+    const int h = it >= per, r = it - h * per;
+    if (r >= N) continue;
+    float2 acc[NK][CO / 2];
 #pragma unroll
-    for (int i = 0; i < C; ++i) acc[i] = 0.0f;
-    const float* gk = g + (int64_t)k * C * N;
+    for (int k = 0; k < NK; ++k)
 #pragma unroll
+      for (int e = 0; e < CO / 2; ++e) acc[k][e] = make_float2(0.0f, 0.0f);
+#pragma unroll 3
     for (int t = 0; t < 9; ++t) {
-      const int rn = nbr[r * 9 + (8 - t)];
-      auto term = [&](int o) {
-        const float v = gk[o * N + rn];
-        const float4* wp = reinterpret_cast<const float4*>(WT + (t * C + o) * C);
+      const float* gr = g + nbr[r * 9 + (8 - t)];
+#pragma unroll 4
+      for (int o = 0; o < C; ++o) {
+        float2 ww[CO / 2];
+        load_half<C>(WT + (t * C + o) * C + h * CO, ww);
 #pragma unroll
-        for (int i4 = 0; i4 < C / 4; ++i4) {
-          const float4 w = wp[i4];
-          acc[4 * i4] = fmaf(v, w.x, acc[4 * i4]);
-          acc[4 * i4 + 1] = fmaf(v, w.y, acc[4 * i4 + 1]);
-          acc[4 * i4 + 2] = fmaf(v, w.z, acc[4 * i4 + 2]);
-          acc[4 * i4 + 3] = fmaf(v, w.w, acc[4 * i4 + 3]);
+        for (int k = 0; k < NK; ++k) {
+          const float v = gr[(k * C + o) * N];
+#pragma unroll
+          for (int e = 0; e < CO / 2; ++e) fma_pair(acc[k][e], make_float2(v, v), ww[e]);
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < CO / 2; ++e) {
+      float v0[NK], v1[NK];
+#pragma unroll
+      for (int k = 0; k < NK; ++k) {
+        v0[k] = acc[k][e].x;
+        v1[k] = acc[k][e].y;
+      }
+      emit(h * CO + 2 * e, r, v0);
+      emit(h * CO + 2 * e + 1, r, v1);
+    }
+  }
+}
+
+// dW[o][i][t] += sum_r g[k][o][r] in[i][nbr(r,t)] and db[o] = sum_r g[k][o][r] for the NK
+// cotangents k, written to the O rows at the layer's parameter offset (reference layout
+// (o, i, ky, kx) then bias). Thread = (cotangent, 2 Q output channels, input channel, half of the
+// sites, in order); it slides a 3 x 3 window along a row, so a site costs 3 window and 2 Q cotangent
+// loads for 18 Q multiply-adds (in packed pairs of outputs). The two halves are summed with a lane
+// shuffle. Q: two pairs of outputs, one where that would leave most of the threads idle.
+template <int C, int NK>
+__device__ inline void weight_grads(const float* __restrict__ g /*[NK][C][N]*/, const float* __restrict__ in /*[cin][N]*/,
+                                    int cin, int L, bool has_bias, float* __restrict__ o_re, float* __restrict__ o_im,
+                                    bool accumulate) {
+  constexpr int Q = C >= 12 ? 2 : 1, G = C / (2 * Q);
+  const int N = L * L, items = NK * G * cin * 2;
+  // every lane of a warp runs the same iterations (kJacThreads is a multiple of 32), so the
+  // full-warp shuffles below always see all 32 lanes; lanes past `items` add zeros
+  for (int base = 0; base < items; base += kJacThreads) {
+    const int it = base + threadIdx.x;
+    const bool active = it < items;
+    const int half = it & 1, rest = active ? it >> 1 : 0;
+    const int i = rest % cin, og = (rest / cin) % G, k = rest / (cin * G);
+    float2 acc[Q][9], bacc[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      bacc[q] = make_float2(0.0f, 0.0f);
+#pragma unroll
+      for (int t = 0; t < 9; ++t) acc[q][t] = make_float2(0.0f, 0.0f);
+    }
+    const float* gk = g + (k * C + 2 * Q * og) * N;
+    const float* ini = in + i * N;
+    const int r0 = half ? N / 2 : 0, r1 = !active ? 0 : (half ? N : N / 2);
+    for (int r = r0; r < r1;) {  // one row, or the half's part of it
+      const int y = r / L, x0 = r - y * L, x1 = min(L, x0 + r1 - r);
+      const float* row[3] = {ini + (y == 0 ? L - 1 : y - 1) * L, ini + y * L, ini + (y == L - 1 ? 0 : y + 1) * L};
+      const float* gy = gk + y * L;
+      float a[3][3];  // window rows and columns x - 1, x, x + 1
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        a[j][0] = row[j][x0 == 0 ? L - 1 : x0 - 1];
+        a[j][1] = row[j][x0];
+      }
+#pragma unroll 2
+      for (int x = x0; x < x1; ++x) {
+        const int xn = x + 1 == L ? 0 : x + 1;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) a[j][2] = row[j][xn];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const float2 gv = make_float2(gy[2 * q * N + x], gy[(2 * q + 1) * N + x]);
+#pragma unroll
+          for (int t = 0; t < 9; ++t) fma_pair(acc[q][t], gv, make_float2(a[t / 3][t % 3], a[t / 3][t % 3]));
+          bacc[q].x += gv.x;
+          bacc[q].y += gv.y;
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          a[j][0] = a[j][1];
+          a[j][1] = a[j][2];
+        }
+      }
+      r += x1 - x0;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        acc[q][t].x += __shfl_xor_sync(0xffffffffu, acc[q][t].x, 1);
+        acc[q][t].y += __shfl_xor_sync(0xffffffffu, acc[q][t].y, 1);
+      }
+      bacc[q].x += __shfl_xor_sync(0xffffffffu, bacc[q].x, 1);
+      bacc[q].y += __shfl_xor_sync(0xffffffffu, bacc[q].y, 1);
+    }
+    float* row_out = k == 0 ? o_re : o_im;
+    if (active && half == 0 && row_out) {
+      auto put = [&](int o, const float (&w)[9], float bias) {
+        float* dst = row_out + ((int64_t)o * cin + i) * 9;
+#pragma unroll
+        for (int t = 0; t < 9; ++t) dst[t] = accumulate ? dst[t] + w[t] : w[t];
+        if (has_bias && i == 0) {
+          float* db = row_out + (int64_t)C * cin * 9 + o;
+          *db = accumulate ? *db + bias : bias;
         }
       };
-      if constexpr (C <= 8) {
-        // left to itself the compiler unrolls all 8 output channels here and spills 4 KB per
-        // thread; four at a time keeps every value in registers
-#pragma unroll 4
-        for (int o = 0; o < C; ++o) term(o);
-      } else {
-        for (int o = 0; o < C; ++o) term(o);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        float w0[9], w1[9];
+#pragma unroll
+        for (int t = 0; t < 9; ++t) {
+          w0[t] = acc[q][t].x;
+          w1[t] = acc[q][t].y;
+        }
+        put(2 * (Q * og + q), w0, bacc[q].x);
+        put(2 * (Q * og + q) + 1, w1, bacc[q].y);
       }
     }
+  }
+}
+
+// One layer's weights on their way to shared memory: loaded into registers before a pass, stored
+// after it, so that the loads' latency is the pass's. T: transposed to [t][o][i] (C inputs).
+template <int C>
+struct JacStage {
+  static constexpr int kFloats = 9 * C * C + C, kPer = (kFloats + kJacThreads - 1) / kJacThreads;
+  float v[kPer];
+  __device__ inline void load(const float* __restrict__ table, int l) {
+    const float* src = table + layer_offset(l, C);
+    const int nf = (int)layer_floats(l, C);
 #pragma unroll
-    for (int i = 0; i < C; ++i)  // constant indices keep acc in registers
-      if (i < cin) gin[((int64_t)k * C + i) * N + r] = acc[i];
+    for (int j = 0; j < kPer; ++j) {
+      const int e = threadIdx.x + j * kJacThreads;
+      v[j] = e < nf ? __ldg(src + e) : 0.0f;
+    }
   }
-}
-
-// stage layer l's table slice into W and its transpose WT[t][o][i]
-template <int C>
-__device__ inline void stage_layer(const float* table, int l, float* W, float* WT) {
-  const int cin = layer_cin(l, C);
-  const float* src = table + layer_offset(l, C);
-  const int nf = cin * 9 * C + C;
-  for (int e = threadIdx.x; e < nf; e += blockDim.x) W[e] = __ldg(src + e);
-  for (int e = threadIdx.x; e < 9 * C * C; e += blockDim.x) {
-    const int t = e / (C * C), o = (e / C) % C, i = e % C;
-    WT[e] = i < cin ? __ldg(src + (i * 9 + t) * C + o) : 0.0f;
+  __device__ inline void load_transposed(const float* __restrict__ table, int l) {
+    const float* src = table + layer_offset(l, C);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int e = threadIdx.x + j * kJacThreads, t = e / (C * C), o = (e / C) % C, i = e % C;
+      v[j] = e < 9 * C * C ? __ldg(src + (i * 9 + t) * C + o) : 0.0f;
+    }
   }
-}
+  __device__ inline void store(float* __restrict__ W) const {
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int e = threadIdx.x + j * kJacThreads;
+      if (e < kFloats) W[e] = v[j];
+    }
+  }
+};
 
-template <int C>
-__global__ void __launch_bounds__(kJacThreads)
+// Shared memory: P and Qa (the layers' inputs), NK cotangents G of X and GA of A (X, which only the
+// forward needs, lies in GA), two weight buffers: 57 KB at L = 10 with 16 channels and both
+// cotangents, three CTAs per SM. One sample per CTA at a time; three barriers per block in the
+// backward, two in the forward. Bound by shared-memory loads and FMA issue: 1.34 ms for 1024 samples
+// at L = 10, 8 blocks, 16 channels, complex (2.31 ms with nine C N buffers, two CTAs per SM, one
+// cotangent per thread in the transposed convolution and nine indexed window loads per site in
+// the weight gradients), 0.58 ms for 2048 at L = 6, 5 blocks, 12 channels (1.25).
+template <int C, int NK>
+__global__ void __launch_bounds__(kJacThreads, 3)
     rc_jacobian_kernel(const float* __restrict__ table, ConvNet net, const uint32_t* __restrict__ spins, int64_t ns,
                        float* __restrict__ o_re, float* __restrict__ o_im, int64_t ldo, float* __restrict__ scratch,
                        SymmJac sj) {
   extern __shared__ float4 smem4[];
   float* sm = reinterpret_cast<float*>(smem4);
-  const int N = net.N, B = net.B, nw = words_for(N);
+  const int L = net.L, N = net.N, B = net.B, nw = words_for(N);
   const int CN = C * N;
-  float* X = sm;                 // [C][N] block input / running activation
-  float* P = X + CN;             // [C][N] pre(X_b)
-  float* Qa = P + CN;            // [C][N] conv1 pre-activation A, then gelu(A)
-  float* G = Qa + CN;            // [2][C][N] cotangent of X
-  float* GA = G + 2 * CN;        // [2][C][N] cotangent of A
-  float* GP = GA + 2 * CN;       // [2][C][N] cotangent of P
-  float* W = GP + 2 * CN;        // layer table slice (C*9*C + C)
-  float* WT = W + C * 9 * C + C; // [9][C][C]
-  int16_t* nbr = reinterpret_cast<int16_t*>(WT + 9 * C * C);
+  float* P = sm;                 // [C][N] pre(X_b)
+  float* Qa = P + CN;            // [C][N] gelu(A_b)
+  float* G = Qa + CN;            // [NK][C][N] cotangent of X
+  float* GA = G + NK * CN;       // [NK][C][N] cotangent of A
+  float* X = GA;                 // [C][N] running activation of the forward
+  float* W0 = GA + NK * CN;      // layer weights, W or WT
+  float* W1 = W0 + JacStage<C>::kFloats;
+  int16_t* nbr = reinterpret_cast<int16_t*>(W1 + JacStage<C>::kFloats);
   __shared__ float red[2][kJacThreads / 32];
-  build_nbr(nbr, net.L);
+  build_nbr(nbr, L);
   float* mine = scratch + (int64_t)blockIdx.x * B * 2 * CN;  // X_b and A_b of every block
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float fs = rsqrtf((float)(B + 1));
   const int cp = net.cplx ? C / 2 : C;
   const int ng = sj.cfg ? sj.nsymm : 1;
+  auto pre_scale = [](int b) { return rsqrtf((float)(b + 1)) * (b == 0 ? 0.70710678118654752f : 1.0f); };
+  JacStage<C> stage;
   for (int64_t smp = blockIdx.x; smp < ns; smp += gridDim.x) {
    for (int g = 0; g < ng; ++g) {
     // v = d log psi_symm / d log psi(T_g s) = w_g psi(T_g s) / psi_symm(s); 1 without symmetry
@@ -856,41 +967,48 @@ __global__ void __launch_bounds__(kJacThreads)
       vr = (float)(wr * ar - wi * ai);
       vi = (float)(wr * ai + wi * ar);
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < N; e += blockDim.x) {
+    stage.load(table, 0);
+    __syncthreads();  // the previous sample's last pass has read P, GA and W0
+    for (int e = threadIdx.x; e < N; e += kJacThreads) {
       const float v = ((src[e >> 5] >> (e & 31)) & 1u) ? 1.0f : -1.0f;
-      for (int c = 0; c < C; ++c) X[c * N + e] = v;
+      for (int c = 0; c < C; ++c) {
+        X[c * N + e] = v;
+        mine[c * N + e] = v;
+      }
+      P[e] = v * pre_scale(0);
     }
+    stage.store(W0);
+    __syncthreads();
     // ---- forward, saving X_b and A_b
     for (int b = 0; b < B; ++b) {
-      const float scale = rsqrtf((float)(b + 1)) * (b == 0 ? 0.70710678118654752f : 1.0f);
-      const int cin = b == 0 ? 1 : C;
-      __syncthreads();
       float* xs = mine + (int64_t)b * 2 * CN;
-      for (int e = threadIdx.x; e < CN; e += blockDim.x) {
-        xs[e] = X[e];
-        const float v = X[e] * scale;
-        if (e < cin * N) P[e] = b == 0 ? v : gelu_tanh(v);
-      }
-      stage_layer<C>(table, 2 * b, W, WT);
+      stage.load(table, 2 * b + 1);
+      conv_sites<C>(P, b == 0 ? 1 : C, W0, nbr, N, [&](int o, int r, float y) {
+        xs[CN + o * N + r] = y;
+        Qa[o * N + r] = gelu_tanh(y);
+      });
+      stage.store(W1);
       __syncthreads();
-      // A = conv1(P) + b1 (pre-activation kept: conv_layer mode 1 on a zeroed buffer)
-      for (int e = threadIdx.x; e < CN; e += blockDim.x) Qa[e] = 0.0f;
+      const bool more = b + 1 < B;
+      if (more) stage.load(table, 2 * b + 2);
+      const float next = pre_scale(b + 1);
+      float* xn = xs + 2 * CN;
+      conv_sites<C>(Qa, C, W1, nbr, N, [&](int o, int r, float y) {
+        const int e = o * N + r;
+        const float x = X[e] + y;
+        X[e] = x;
+        if (more) {
+          xn[e] = x;
+          P[e] = gelu_tanh(x * next);
+        }
+      });
+      if (more) stage.store(W0);
       __syncthreads();
-      conv_layer<C, 1>(P, cin, Qa, W, nbr, N, 1, 1, C * N);
-      __syncthreads();
-      for (int e = threadIdx.x; e < CN; e += blockDim.x) {
-        xs[CN + e] = Qa[e];
-        Qa[e] = gelu_tanh(Qa[e]);
-      }
-      stage_layer<C>(table, 2 * b + 1, W, WT);
-      __syncthreads();
-      conv_layer<C, 1>(Qa, C, X, W, nbr, N, 1, 1, C * N);
     }
-    __syncthreads();
+    stage.load_transposed(table, 2 * B - 1);
     // ---- output cotangents: w_e = f'(z_e) / sum f, f = exp (exp_by_scale) or sinh + 1
     float m = -INFINITY;
-    for (int e = threadIdx.x; e < cp * N; e += blockDim.x) m = fmaxf(m, net.sinhp1 ? fabsf(X[e] * fs) : X[e] * fs);
+    for (int e = threadIdx.x; e < cp * N; e += kJacThreads) m = fmaxf(m, net.sinhp1 ? fabsf(X[e] * fs) : X[e] * fs);
     m = warp_max(m);
     if (lane == 0) red[0][warp] = m;
     __syncthreads();
@@ -898,7 +1016,7 @@ __global__ void __launch_bounds__(kJacThreads)
     for (int w = 1; w < kJacThreads / 32; ++w) m = fmaxf(m, red[0][w]);
     __syncthreads();
     float sr = 0.0f, si = 0.0f;
-    for (int e = threadIdx.x; e < cp * N; e += blockDim.x) {
+    for (int e = threadIdx.x; e < cp * N; e += kJacThreads) {
       if (net.sinhp1) {
         float fr, fi, gr, gi;
         sinhp1_shifted(X[e] * fs, net.cplx ? X[cp * N + e] * fs : 0.0f, m, net.cplx, &fr, &fi, &gr, &gi);
@@ -928,7 +1046,7 @@ __global__ void __launch_bounds__(kJacThreads)
     // 1 / (sr + i si)
     const float den = sr * sr + si * si;
     const float ir = sr / den, ii = -si / den;
-    for (int e = threadIdx.x; e < cp * N; e += blockDim.x) {
+    for (int e = threadIdx.x; e < cp * N; e += kJacThreads) {
       float ar, ai;
       if (net.sinhp1) {
         float fr, fi;
@@ -940,21 +1058,19 @@ __global__ void __launch_bounds__(kJacThreads)
         ar = ex * cs;
         ai = ex * sn;
       }
-      const float ur = ar * ir - ai * ii, ui = ar * ii + ai * ir;  // f'(z) / sum f
-      const float wr = vr * ur - vi * ui, wi = vr * ui + vi * ur;  // times v
-      if (net.cplx) {
-        G[e] = wr * fs;               // d Re / d y_c
-        G[cp * N + e] = -wi * fs;     // d Re / d y_{c+C/2}
-        G[CN + e] = wi * fs;          // d Im / d y_c
-        G[CN + cp * N + e] = wr * fs; // d Im / d y_{c+C/2}
-      } else {
-        G[e] = wr * fs;
-        G[CN + e] = 0.0f;
+      // f'(z) / sum f, then times v (contracted in a fixed way, whatever the code around)
+      const float ur = fmaf(ar, ir, -(ai * ii)), ui = fmaf(ar, ii, ai * ir);
+      const float wr = fmaf(vr, ur, -(vi * ui)), wi = fmaf(vr, ui, vi * ur);
+      G[e] = wr * fs;                                              // d Re / d y_c
+      if (net.cplx) G[cp * N + e] = -wi * fs;                      // d Re / d y_{c+C/2}
+      if (NK == 2) {
+        G[CN + e] = net.cplx ? wi * fs : 0.0f;                     // d Im / d y_c
+        if (net.cplx) G[CN + cp * N + e] = wr * fs;                // d Im / d y_{c+C/2}
       }
     }
     // ---- backward
     float* row_re = o_re + smp * ldo;
-    float* row_im = o_im ? o_im + smp * ldo : nullptr;
+    float* row_im = NK == 2 ? o_im + smp * ldo : nullptr;
     int64_t poff = nparams_rc(B, C);
     for (int b = B - 1; b >= 0; --b) {
       const int cin = b == 0 ? 1 : C;
@@ -962,46 +1078,52 @@ __global__ void __launch_bounds__(kJacThreads)
       const int64_t n2 = (int64_t)C * C * 9 + (last ? 0 : C);
       const int64_t n1 = (int64_t)C * cin * 9 + C;
       poff -= n1 + n2;
-      const float scale = rsqrtf((float)(b + 1)) * (b == 0 ? 0.70710678118654752f : 1.0f);
+      const float scale = pre_scale(b);
       const float* xs = mine + (int64_t)b * 2 * CN;
-      __syncthreads();
-      for (int e = threadIdx.x; e < CN; e += blockDim.x) {
-        const float a = xs[CN + e];
-        Qa[e] = gelu_tanh(a);
-        const float v = xs[e] * scale;
-        if (e < cin * N) P[e] = b == 0 ? v : gelu_tanh(v);
-      }
-      stage_layer<C>(table, 2 * b + 1, W, WT);
-      __syncthreads();
-      // conv2: grads of W2, b2 and of Q (into GA)
-      weight_grads<C>(G, Qa, C, nbr, N, !last, row_re + poff + n1, row_im ? row_im + poff + n1 : nullptr, g > 0);
-      input_grads<C>(G, WT, C, nbr, N, GA);
-      __syncthreads();
-      for (int e = threadIdx.x; e < 2 * CN; e += blockDim.x) GA[e] *= gelu_tanh_grad(xs[CN + (e % CN)]);
-      stage_layer<C>(table, 2 * b, W, WT);
-      __syncthreads();
-      weight_grads<C>(GA, P, cin, nbr, N, true, row_re + poff, row_im ? row_im + poff : nullptr, g > 0);
-      if (b > 0) {
-        input_grads<C>(GA, WT, cin, nbr, N, GP);
-        __syncthreads();
-        for (int e = threadIdx.x; e < 2 * CN; e += blockDim.x) {
-          const int ee = e % CN;
-          G[e] += GP[e] * gelu_tanh_grad(xs[ee] * scale) * scale;
+      // the last block's are still in P and Qa from the forward
+      if (!last) {
+        for (int e = threadIdx.x; e < CN; e += kJacThreads) {
+          Qa[e] = gelu_tanh(xs[CN + e]);
+          const float v = xs[e] * scale;
+          if (e < cin * N) P[e] = b == 0 ? v : gelu_tanh(v);
         }
+      }
+      stage.store(W1);
+      __syncthreads();
+      // conv2: grads of W2, b2 and of A (into GA: those of gelu(A), times its derivative)
+      if (b > 0) stage.load_transposed(table, 2 * b);
+      weight_grads<C, NK>(G, Qa, C, L, !last, row_re + poff + n1, row_im ? row_im + poff + n1 : nullptr, g > 0);
+      input_grads<C, NK>(G, W1, nbr, N, [&](int i, int r, const float (&v)[NK]) {
+        const float d = gelu_tanh_grad(xs[CN + i * N + r]);
+#pragma unroll
+        for (int k = 0; k < NK; ++k) GA[k * CN + i * N + r] = v[k] * d;
+      });
+      if (b > 0) stage.store(W0);
+      __syncthreads();
+      if (b > 0) stage.load_transposed(table, 2 * b - 1);
+      weight_grads<C, NK>(GA, P, cin, L, true, row_re + poff, row_im ? row_im + poff : nullptr, g > 0);
+      if (b > 0) {
+        input_grads<C, NK>(GA, W0, nbr, N, [&](int i, int r, const float (&v)[NK]) {
+          const float d = gelu_tanh_grad(xs[i * N + r] * scale);
+#pragma unroll
+          for (int k = 0; k < NK; ++k) G[k * CN + i * N + r] += v[k] * d * scale;
+        });
+        __syncthreads();  // G is complete; P, Qa and W1 have been read
       }
     }
    }
   }
 }
 
-template <int C>
-int launch_jacobian_c(const float* table, const ConvNet& net, const uint32_t* spins, int64_t ns, float* o_re,
+template <int C, int NK>
+int launch_jacobian_k(const float* table, const ConvNet& net, const uint32_t* spins, int64_t ns, float* o_re,
                       float* o_im, int64_t ldo, float* scratch, int64_t scratch_floats, const SymmJac& sj,
                       cudaStream_t st) {
   const int CN = C * net.N;
-  const int64_t sf = 3LL * CN + 6LL * CN + C * 9 * C + C + 9 * C * C;
+  const int64_t sf = 2LL * CN + 2LL * NK * CN + 2 * JacStage<C>::kFloats;
   const int smem = (int)(sf * 4 + net.N * 9 * 2 + 16);
-  auto k = rc_jacobian_kernel<C>;
+  if (smem > device_max_smem_optin()) return QGX_ERR_UNSUPPORTED;
+  auto k = rc_jacobian_kernel<C, NK>;
   if (smem > 48 * 1024) QGX_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int per_sm = 0;
   QGX_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kJacThreads, smem));
@@ -1012,6 +1134,15 @@ int launch_jacobian_c(const float* table, const ConvNet& net, const uint32_t* sp
   if (grid < 1) return QGX_ERR_ARG;
   k<<<(unsigned)grid, kJacThreads, smem, st>>>(table, net, spins, ns, o_re, o_im, ldo, scratch, sj);
   return launch_status();
+}
+
+// one cotangent where nobody takes the imaginary rows
+template <int C>
+int launch_jacobian_c(const float* table, const ConvNet& net, const uint32_t* spins, int64_t ns, float* o_re,
+                      float* o_im, int64_t ldo, float* scratch, int64_t scratch_floats, const SymmJac& sj,
+                      cudaStream_t st) {
+  return o_im ? launch_jacobian_k<C, 2>(table, net, spins, ns, o_re, o_im, ldo, scratch, scratch_floats, sj, st)
+              : launch_jacobian_k<C, 1>(table, net, spins, ns, o_re, o_im, ldo, scratch, scratch_floats, sj, st);
 }
 
 // shared memory of the FP32 forward with S samples per CTA, in the blocked order (blk, even L
