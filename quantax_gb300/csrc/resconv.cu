@@ -88,8 +88,29 @@ __global__ void rc_prepare_kernel(const float* __restrict__ params, int B, int C
   }
 }
 
-__device__ inline void stage_floats(float* dst, const float* src, int64_t n) {
-  for (int64_t e = threadIdx.x; e < n; e += blockDim.x) dst[e] = __ldg(src + e);
+// One layer's n weights and biases (n a multiple of 4, at most 9 C C + C) to shared memory: the
+// loads of a thread all go out before its first store, 16 bytes each (2.34 against 2.44 ms per 16384
+// forwards at L = 10, 8 blocks, 16 channels with single floats and prefetches to L1 a layer ahead;
+// no staging at all would give 2.31); a table that does not start on 16 bytes goes float by float.
+template <int C>
+__device__ inline void stage_layer(float* dst, const float* src, int n) {
+  if ((reinterpret_cast<uintptr_t>(src) & 15) != 0) {
+    for (int e = threadIdx.x; e < n; e += kFwdThreads) dst[e] = __ldg(src + e);
+    return;
+  }
+  constexpr int kPer = ((9 * C * C + C) / 4 + kFwdThreads - 1) / kFwdThreads;
+  const float4* s4 = reinterpret_cast<const float4*>(src);
+  float4 v[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int e = threadIdx.x + k * kFwdThreads;
+    if (e < n / 4) v[k] = __ldg(s4 + e);
+  }
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int e = threadIdx.x + k * kFwdThreads;
+    if (e < n / 4) reinterpret_cast<float4*>(dst)[e] = v[k];
+  }
 }
 
 // Floats between consecutive samples' activations in the forward's shared memory: C N padded to
@@ -127,6 +148,17 @@ __device__ inline void fma_pair(float2& c, float2 a, float2 b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(cc));
 }
 
+// A float at a 32-bit shared-memory address. The convolutions keep the neighbours of a thread's
+// sites as such addresses, so that a gather is one 32-bit addition (of the input channel's offset)
+// and a load; through 64-bit pointers the compiler's address arithmetic took issue slots and
+// registers from the multiply-adds (2.58 against 2.44 ms per 16384 forwards at L = 10, 8 blocks,
+// 16 channels).
+__device__ inline float ld_shared(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+
 // out[a][o][r] = act(sum_{i,tap} W[i][tap][o] in[a][i][nbr(r,tap)] + bias[o]); mode 0: gelu and store,
 // mode 1: accumulate into out (residual add). A thread computes the C outputs of SPT sites
 // r = g + k G (G = ceil(N / SPT)), so consecutive threads gather consecutive sites (no bank
@@ -141,28 +173,28 @@ __device__ inline void conv_layer(const float* __restrict__ in, int cin, float* 
   for (int it = threadIdx.x; it < S * G; it += blockDim.x) {
     const int a = it / G, g = it - a * G;
     int r[SPT];
-    int nb[SPT][9];
+    uint32_t nb[SPT][9];  // byte offsets of the neighbours in input channel 0
 #pragma unroll
     for (int k = 0; k < SPT; ++k) {
       r[k] = g + k * G;
       const int rc = r[k] < N ? r[k] : N - 1;  // a site past the end reads a valid one, is not stored
 #pragma unroll
-      for (int t = 0; t < 9; ++t) nb[k][t] = nbr[rc * 9 + t];
+      for (int t = 0; t < 9; ++t) nb[k][t] = 4u * (uint32_t)(nbr[rc * 9 + t] + a * ss);
     }
     float2 acc[SPT][C / 2];  // output channels (2 h, 2 h + 1)
 #pragma unroll
     for (int k = 0; k < SPT; ++k)
 #pragma unroll
       for (int h = 0; h < C / 2; ++h) acc[k][h] = make_float2(bias[2 * h], bias[2 * h + 1]);
-    const float* ina = in + (int64_t)a * ss;
+    const uint32_t in_s = (uint32_t)__cvta_generic_to_shared(in);
     for (int i = 0; i < cin; ++i) {
-      const float* ini = ina + i * N;
+      const uint32_t ini = in_s + 4u * (uint32_t)(i * N);
 #pragma unroll
       for (int t = 0; t < 9; ++t) {
         float2 v[SPT];
 #pragma unroll
         for (int k = 0; k < SPT; ++k) {
-          const float x = ini[nb[k][t]];
+          const float x = ld_shared(nb[k][t] + ini);
           v[k] = make_float2(x, x);
         }
         const float4* wp = reinterpret_cast<const float4*>(w + (i * 9 + t) * C);
@@ -210,8 +242,9 @@ __device__ inline void conv_layer(const float* __restrict__ in, int cin, float* 
 // is also written as the next block's pre-activation pnext = gelu(x pscale) (the separate pass
 // of the site-order kernel, the same floats). CIN > 0 fixes the input channel count at compile
 // time (the C-channel layers); the input-channel loop is unrolled four times either way
-// (measured: 2.77 ms per 16384 forwards at L = 10 against 2.93 without; eight and sixteen were
-// slower).
+// (2.34 ms per 16384 forwards at L = 10, 8 blocks; two times 2.40, eight no faster, sixteen slower).
+// Bound by the multiply-add pipe and what does not overlap it: 2.07 ms without staging and GELU,
+// where these operands and loads alone run at 109 of 128 multiply-adds per clock and SM (1.74 ms).
 template <int C, int CO, int CIN = 0>
 __device__ inline void conv_layer_blocked(const float* __restrict__ in, int cin_rt, float* __restrict__ out,
                                           const float* __restrict__ w, const int16_t* __restrict__ nbr, int N,
@@ -229,21 +262,21 @@ __device__ inline void conv_layer_blocked(const float* __restrict__ in, int cin_
     if (j >= items) continue;
     const int a = j / NB, g = j - a * NB;
     const int o0 = h * CO;
-    int nb[16];
+    uint32_t nb[16];  // byte offsets of the patch in input channel 0
 #pragma unroll
-    for (int k = 0; k < 16; ++k) nb[k] = nbr[g * 16 + k];
+    for (int k = 0; k < 16; ++k) nb[k] = 4u * (uint32_t)(nbr[g * 16 + k] + a * ss);
     float2 acc[4][CO / 2];  // block position q = 2 py + px; output channels (o0 + 2 e, o0 + 2 e + 1)
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
       for (int e = 0; e < CO / 2; ++e) acc[q][e] = make_float2(bias[o0 + 2 * e], bias[o0 + 2 * e + 1]);
-    const float* ina = in + (int64_t)a * ss;
+    const uint32_t in_s = (uint32_t)__cvta_generic_to_shared(in);
 #pragma unroll 4
     for (int i = 0; i < cin; ++i) {
-      const float* ini = ina + i * N;
+      const uint32_t ini = in_s + 4u * (uint32_t)(i * N);
       float d[16];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) d[k] = ini[nb[k]];
+      for (int k = 0; k < 16; ++k) d[k] = ld_shared(nb[k] + ini);
 #pragma unroll
       for (int t = 0; t < 9; ++t) {
         const int dy = t / 3, dx = t % 3;
@@ -288,18 +321,6 @@ __device__ inline void conv_layer_blocked(const float* __restrict__ in, int cin_
         }
       }
     }
-  }
-}
-
-// Asks L1 for the 128-byte lines of the n floats at src, one prefetch per line, every address
-// inside [src, src + n). Issued for the next layer's weights before a convolution, so that the
-// staging after it reads L1 rather than L2.
-__device__ inline void prefetch_l1(const float* src, int64_t n) {
-  const size_t a0 = __cvta_generic_to_global(src), a1 = __cvta_generic_to_global(src + n);
-  for (size_t k = threadIdx.x;; k += blockDim.x) {
-    const size_t a = k == 0 ? a0 : (a0 & ~size_t(127)) + 128 * k;
-    if (a >= a1) break;
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
   }
 }
 
@@ -357,11 +378,12 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
   float* Wl = sm + rc_weights_offset(S, SS);  // 16-byte aligned: the weights are read as float4
   int16_t* nbr = reinterpret_cast<int16_t*>(Wl + C * 9 * C + C);
   int16_t* site = nbr + (BLK ? N * 4 : 0);  // blocked index of each site (BLK only)
+  const int64_t total = n_live ? min(ncfg, *n_live) : ncfg;
+  if ((int64_t)blockIdx.x * S >= total) return;
   if (BLK)
     build_blocked_tables(nbr, site, net.L);
   else
     build_nbr(nbr, net.L);
-  const int64_t total = n_live ? min(ncfg, *n_live) : ncfg;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int64_t base = (int64_t)blockIdx.x * S; base < total; base += (int64_t)gridDim.x * S) {
     const int s_here = (int)(total - base < S ? total - base : S);
@@ -384,8 +406,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
           P[(int64_t)a * SS + rem] = b == 0 ? v : gelu_tanh(v);
         }
       }
-      stage_floats(Wl, table + layer_offset(2 * b, C), layer_floats(2 * b, C));
-      if (BLK) prefetch_l1(table + layer_offset(2 * b + 1, C), layer_floats(2 * b + 1, C));
+      stage_layer<C>(Wl, table + layer_offset(2 * b, C), (int)layer_floats(2 * b, C));
       __syncthreads();
       if (BLK && cin == C)
         conv_layer_blocked<C, rc_blocked_co<C>(), C>(P, C, Q, Wl, nbr, N, S, 0, SS);
@@ -394,10 +415,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
       else
         conv_layer<C, kFwdSPT>(P, cin, Q, Wl, nbr, N, S, 0, SS);
       __syncthreads();
-      stage_floats(Wl, table + layer_offset(2 * b + 1, C), layer_floats(2 * b + 1, C));
-      // the next layer in order: the next block's first convolution, or block 0's for the next samples
-      const int lnext = b + 1 < net.B ? 2 * b + 2 : 0;
-      if (BLK) prefetch_l1(table + layer_offset(lnext, C), layer_floats(lnext, C));
+      stage_layer<C>(Wl, table + layer_offset(2 * b + 1, C), (int)layer_floats(2 * b + 1, C));
       __syncthreads();
       if (BLK)
         conv_layer_blocked<C, rc_blocked_co<C>(), C>(Q, C, X, Wl, nbr, N, S, 1, SS, b + 1 < net.B ? P : nullptr,
@@ -1202,8 +1220,12 @@ int launch_forward_c(const float* table, const ConvNet& net, const uint32_t* cfg
   int per_sm = 0;
   QGX_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kFwdThreads, smem));
   if (per_sm < 1) return QGX_ERR_UNSUPPORTED;
+  // One CTA per S configurations, in the hardware's order, not a resident set that strides: two
+  // CTAs of an SM do not advance evenly, and with a fixed share each the faster one leaves the
+  // other alone at the end (13.4 of 16 warps active on average; 2.77 -> 2.57 ms per 16384 forwards
+  // at L = 10, 8 blocks, 16 channels).
   const int64_t want = (ncfg + S - 1) / S;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)device_sm_count() * per_sm, want));
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(INT32_MAX, want));
   k<<<grid, kFwdThreads, smem, st>>>(table, net, cfg, ncfg, n_live, out, S);
   return launch_status();
 }
