@@ -323,15 +323,127 @@ __global__ void __launch_bounds__(NT, 1)
 }
 
 // ---------------------------------------------------------------------------------------
-// Local energies: one warp per sample, connected configurations generated in-kernel.
-__device__ inline int bit_of(const uint32_t* sp, int k) { return (int)((sp[k >> 5] >> (k & 31)) & 1u); }
+// Local energies: a warp takes NS samples at a time, connected configurations are generated in the
+// kernel. Lane l of the warp holds word l of the packed configurations, and one term of 32
+// consecutive terms of the operator: its site, spin and matrix element, and later the log ratio of
+// its connected configuration. Two things bound it:
+// - An FP64 instruction takes the same 64 clocks of a sub-core for one lane as for 32, and exp is
+//   about 25 of them: the exponentials are taken by the lanes side by side, each adding to a partial
+//   sum of its own (summed over the warp at the end). One exponential and one comparison per
+//   configuration in lane 0 were the whole time before.
+// - The rows of C and S, from shared memory or L2, are read once for NS samples.
+// 4096 samples, n = 128, m = 512: 640 -> 111 us; 8192, n = 64, m = 256: 597 -> 65 us.
 
-template <int JT, bool SMEM, int NT>
+// whether spin k of the configuration in `word` (word l in lane l) is up; k may differ by lane
+__device__ inline bool spin_up(uint32_t word, int k) {
+  return (__shfl_sync(kFull, word, k >> 5) >> (k & 31)) & 1u;
+}
+
+// compute_theta of NS configurations held as words, reading every row of W once (the same sums)
+template <int JT, int NS>
+__device__ inline void theta_rows(const RbmTable& T, int n, int mp, const uint32_t (&word)[NS], int lane,
+                                  float (&th)[NS][JT][4]) {
+#pragma unroll
+  for (int j = 0; j < JT; ++j) {
+    const float4 bv = *reinterpret_cast<const float4*>(T.b + 128 * j + 4 * lane);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      th[s][j][0] = bv.x;
+      th[s][j][1] = bv.y;
+      th[s][j][2] = bv.z;
+      th[s][j][3] = bv.w;
+    }
+  }
+  for (int k0 = 0; k0 < n; k0 += 32) {
+    uint32_t w[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) w[s] = __shfl_sync(kFull, word[s], k0 >> 5);
+    const int kn = n - k0 < 32 ? n - k0 : 32;
+#pragma unroll 2
+    for (int k = 0; k < kn; ++k) {
+#pragma unroll
+      for (int j = 0; j < JT; ++j) {
+        const float4 wv = *reinterpret_cast<const float4*>(T.Wt + (int64_t)(k0 + k) * mp + 128 * j + 4 * lane);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+          const float sk = ((w[s] >> k) & 1u) ? 1.0f : -1.0f;
+          th[s][j][0] = fmaf(sk, wv.x, th[s][j][0]);
+          th[s][j][1] = fmaf(sk, wv.y, th[s][j][1]);
+          th[s][j][2] = fmaf(sk, wv.z, th[s][j][2]);
+          th[s][j][3] = fmaf(sk, wv.w, th[s][j][3]);
+        }
+      }
+    }
+  }
+}
+
+// (a.x b.x, a.y b.y) and (a.x b.x + c.x, a.y b.y + c.y) in one instruction, rounded as the two
+// scalar ones
+__device__ inline float2 mul_pair(float2 a, float2 b) {
+  float2 c;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(c.x), "=f"(c.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return c;
+}
+__device__ inline float2 fma_pair(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
+// lane_log_flip1 of NS samples for flipping site k (up: its spin in each), one read of the row;
+// the same operations and products per sample
+template <int JT, int NS>
+__device__ inline void lane_log_flip1_rows(const RbmTable& T, int mp, int k, const bool (&up)[NS],
+                                           const float (&t)[NS][JT][4], int lane, float (&lg)[NS]) {
+  float prod[NS];
+#pragma unroll
+  for (int s = 0; s < NS; ++s) prod[s] = 1.0f;
+#pragma unroll
+  for (int j = 0; j < JT; ++j) {
+    const float4 cv = *reinterpret_cast<const float4*>(T.C + (int64_t)k * mp + 128 * j + 4 * lane);
+    const float4 sv = *reinterpret_cast<const float4*>(T.S + (int64_t)k * mp + 128 * j + 4 * lane);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const float m = up[s] ? -1.0f : 1.0f;
+      const float2 m2 = make_float2(m, m);
+      const float2 lo = fma_pair(mul_pair(m2, make_float2(t[s][j][0], t[s][j][1])), make_float2(sv.x, sv.y),
+                                 make_float2(cv.x, cv.y));
+      const float2 hi = fma_pair(mul_pair(m2, make_float2(t[s][j][2], t[s][j][3])), make_float2(sv.z, sv.w),
+                                 make_float2(cv.z, cv.w));
+      prod[s] *= lo.x;
+      prod[s] *= lo.y;
+      prod[s] *= hi.x;
+      prod[s] *= hi.y;
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < NS; ++s) lg[s] = logf(prod[s]);
+}
+
+// The warp sums of four values, by the additions of warp_sum (partners 16, 8, 4, 2, 1 lanes away),
+// the first two exchanges carrying two values each; value q in lane sum4_lane(q)
+__device__ inline float warp_sum4(const float (&v)[4], int lane) {
+  const bool h = lane & 16, g = lane & 8;
+  const float a = (h ? v[1] : v[0]) + __shfl_xor_sync(kFull, h ? v[0] : v[1], 16);
+  const float b = (h ? v[3] : v[2]) + __shfl_xor_sync(kFull, h ? v[2] : v[3], 16);
+  float s = (g ? b : a) + __shfl_xor_sync(kFull, g ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+  return s;
+}
+__device__ inline int sum4_lane(int q) { return ((q & 1) << 4) | ((q & 2) << 2); }
+
+template <int JT, bool SMEM, int NT, int NS>
 __device__ inline void eloc_body(float* sm, const float* __restrict__ table, int n, int mp, const qgx_operator_t& op,
                                  const uint32_t* __restrict__ spins, int64_t ns, double* __restrict__ eloc,
                                  int64_t table_nf, int cta, int nctas) {
   constexpr int kWarps = NT / 32;
-  uint32_t* sp_all = reinterpret_cast<uint32_t*>(sm + (SMEM ? table_nf : 0));
   RbmTable T;
   if (SMEM) {
     stage(sm, table, table_nf);
@@ -341,58 +453,128 @@ __device__ inline void eloc_body(float* sm, const float* __restrict__ table, int
     T = table_view(table, n, mp);
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t* sp = sp_all + 32 * warp;
   const int nw = words_for(n);
   for (int64_t slot = warp;; slot += kWarps) {
-    const int64_t c = slot * nctas + cta;
-    if (c >= ns) break;
-    if (lane < nw) sp[lane] = spins[c * nw + lane];
-    __syncwarp();
-    float th[JT][4], t[JT][4];
-    compute_theta<JT>(T, n, mp, sp, lane, th);
+    const int64_t c0 = (slot * nctas + cta) * NS;
+    if (c0 >= ns) break;
+    uint32_t word[NS];
 #pragma unroll
-    for (int j = 0; j < JT; ++j)
+    for (int s = 0; s < NS; ++s) {
+      const int64_t c = c0 + s < ns ? c0 + s : ns - 1;  // past the end: the last sample again, not stored
+      word[s] = lane < nw ? spins[c * nw + lane] : 0u;
+    }
+    float t[NS][JT][4];
+    theta_rows<JT, NS>(T, n, mp, word, lane, t);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) t[j][q] = tanhf(th[j][q]);
+    for (int s = 0; s < NS; ++s)
+#pragma unroll
+      for (int j = 0; j < JT; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) t[s][j][q] = tanhf(t[s][j][q]);
 
-    double ed = 0.0;
-    for (int k = lane; k < op.n_z; k += 32) ed += op.z_J[k] * (double)spin_at(sp, op.z_i[k]);
-    for (int k = lane; k < op.n_zz; k += 32)
-      ed += op.zz_J[k] * (double)(spin_at(sp, op.zz_ij[2 * k]) * spin_at(sp, op.zz_ij[2 * k + 1]));
-    ed = warp_sum(ed);
+    double ed[NS], eo[NS];  // this lane's parts of the diagonal and off-diagonal sums
+#pragma unroll
+    for (int s = 0; s < NS; ++s) ed[s] = eo[s] = 0.0;
+    for (int k0 = 0; k0 < op.n_z; k0 += 32) {
+      const bool in = k0 + lane < op.n_z;
+      const int i = in ? op.z_i[k0 + lane] : 0;
+      const double J = in ? op.z_J[k0 + lane] : 0.0;
+#pragma unroll
+      for (int s = 0; s < NS; ++s) ed[s] += spin_up(word[s], i) ? J : -J;
+    }
+    for (int k0 = 0; k0 < op.n_zz; k0 += 32) {
+      const bool in = k0 + lane < op.n_zz;
+      const int i = in ? op.zz_ij[2 * (k0 + lane)] : 0, j = in ? op.zz_ij[2 * (k0 + lane) + 1] : 0;
+      const double J = in ? op.zz_J[k0 + lane] : 0.0;
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const bool bi = spin_up(word[s], i), bj = spin_up(word[s], j);
+        ed[s] += bi == bj ? J : -J;
+      }
+    }
 
-    double eo = 0.0;  // accumulated in lane 0
-    for (int k = 0; k < op.n_f1; ++k) {
-      const int site = op.f1_i[k];
-      const int bs = bit_of(sp, site);
-      const double elem = op.f1_J[2 * k + bs];
-      if (elem == 0.0) continue;
-      const float sk = bs ? 1.0f : -1.0f;
-      const float l = warp_sum(lane_log_flip1<JT>(T, mp, site, sk, t, lane)) - 2.0f * sk * T.a[site];
-      if (lane == 0) eo += elem * exp((double)l);
+    for (int k0 = 0; k0 < op.n_f1; k0 += 32) {
+      const bool in = k0 + lane < op.n_f1;
+      const int site = in ? op.f1_i[k0 + lane] : 0;
+      uint32_t ups[NS], live = 0;
+      double elem[NS];
+      float sum[NS];
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const bool up = spin_up(word[s], site);
+        ups[s] = __ballot_sync(kFull, up);
+        elem[s] = in ? op.f1_J[2 * (k0 + lane) + up] : 0.0;
+        live |= __ballot_sync(kFull, elem[s] != 0.0);
+        sum[s] = 0.0f;
+      }
+      while (live) {  // four configurations at a time
+        float lg[NS][4];
+        int mine = -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float l[NS];
+#pragma unroll
+          for (int s = 0; s < NS; ++s) l[s] = 0.0f;
+          if (live) {
+            const int e = __ffs(live) - 1;
+            live &= live - 1;
+            if (lane == e) mine = q;
+            bool up[NS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) up[s] = (ups[s] >> e) & 1u;
+            lane_log_flip1_rows<JT, NS>(T, mp, __shfl_sync(kFull, site, e), up, t, lane, l);
+          }
+#pragma unroll
+          for (int s = 0; s < NS; ++s) lg[s][q] = l[s];
+        }
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+          const float v = __shfl_sync(kFull, warp_sum4(lg[s], lane), sum4_lane(mine < 0 ? 0 : mine));
+          if (mine >= 0) sum[s] = v;
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const float sk = ((ups[s] >> lane) & 1u) ? 1.0f : -1.0f;
+        const float l = sum[s] - 2.0f * sk * T.a[site];
+        if (elem[s] != 0.0) eo[s] += elem[s] * exp((double)l);
+      }
     }
-    for (int k = 0; k < op.n_f2; ++k) {
-      const int i = op.f2_ij[2 * k], j = op.f2_ij[2 * k + 1];
-      const int bi = bit_of(sp, i), bj = bit_of(sp, j);
-      const double elem = op.f2_J[4 * k + 2 * bi + bj];
-      if (elem == 0.0) continue;
-      const float si = bi ? 1.0f : -1.0f, sj = bj ? 1.0f : -1.0f;
-      float d[JT][4];
-      const float l = warp_sum(lane_log_flip2<JT>(T, mp, i, si, j, sj, t, lane, d)) -
-                      2.0f * (si * T.a[i] + sj * T.a[j]);
-      if (lane == 0) eo += elem * exp((double)l);
+    for (int k0 = 0; k0 < op.n_f2; k0 += 32) {
+      const bool in = k0 + lane < op.n_f2;
+      const int i = in ? op.f2_ij[2 * (k0 + lane)] : 0, j = in ? op.f2_ij[2 * (k0 + lane) + 1] : 0;
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const bool bi = spin_up(word[s], i), bj = spin_up(word[s], j);
+        const double elem = in ? op.f2_J[4 * (k0 + lane) + 2 * bi + bj] : 0.0;
+        const float si = bi ? 1.0f : -1.0f, sj = bj ? 1.0f : -1.0f;
+        float sum = 0.0f;
+        for (uint32_t live = __ballot_sync(kFull, elem != 0.0); live; live &= live - 1) {
+          const int e = __ffs(live) - 1;
+          float d[JT][4];
+          const float l = warp_sum(lane_log_flip2<JT>(T, mp, __shfl_sync(kFull, i, e), __shfl_sync(kFull, si, e),
+                                                      __shfl_sync(kFull, j, e), __shfl_sync(kFull, sj, e), t[s], lane,
+                                                      d));
+          if (lane == e) sum = l;
+        }
+        const float l = sum - 2.0f * (si * T.a[i] + sj * T.a[j]);
+        if (elem != 0.0) eo[s] += elem * exp((double)l);
+      }
     }
-    if (lane == 0) eloc[c] = op.c0 + ed + eo;
-    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const double e = op.c0 + warp_sum(ed[s]) + warp_sum(eo[s]);
+      if (lane == 0 && c0 + s < ns) eloc[c0 + s] = e;
+    }
   }
 }
 
-template <int JT, bool SMEM, int NT>
+template <int JT, bool SMEM, int NT, int NS>
 __global__ void __launch_bounds__(NT, 1)
     eloc_kernel(const float* __restrict__ table, int n, int mp, qgx_operator_t op, const uint32_t* __restrict__ spins,
                 int64_t ns, double* __restrict__ eloc, int64_t table_nf) {
   extern __shared__ float4 smem4[];
-  eloc_body<JT, SMEM, NT>(reinterpret_cast<float*>(smem4), table, n, mp, op, spins, ns, eloc, table_nf, blockIdx.x,
+  eloc_body<JT, SMEM, NT, NS>(reinterpret_cast<float*>(smem4), table, n, mp, op, spins, ns, eloc, table_nf, blockIdx.x,
                           gridDim.x);
 }
 
@@ -458,7 +640,7 @@ __global__ void __launch_bounds__(NT, 1) eloc_batch_kernel(const __grid_constant
   extern __shared__ float4 smem4[];
   const int j = batch_job_of(b.cta0, b.njobs);
   const ElocJob& J = b.job[j];
-  eloc_body<JT, SMEM, NT>(reinterpret_cast<float*>(smem4), J.table, J.n, J.mp, J.op, J.spins, J.ns, J.eloc, J.table_nf,
+  eloc_body<JT, SMEM, NT, 1>(reinterpret_cast<float*>(smem4), J.table, J.n, J.mp, J.op, J.spins, J.ns, J.eloc, J.table_nf,
                           (int)blockIdx.x - b.cta0[j], b.cta0[j + 1] - b.cta0[j]);
 }
 
@@ -797,22 +979,31 @@ int launch_sweep(const float* table, int n, int mp, uint32_t* spins, float* log_
                                                                     seed, step0, reweight, nbr, z, hop, smem, st);
 }
 
+template <int JT, bool SMEM, int NS>
+int launch_eloc_v(const float* table, int n, int mp, const qgx_operator_t& op, const uint32_t* spins, int64_t ns,
+                  double* eloc, size_t smem, cudaStream_t st) {
+  constexpr int NT = threads_for<JT>();
+  auto k = eloc_kernel<JT, SMEM, NT, NS>;
+  int grid, rc;
+  if ((rc = configure(k, NT, smem, (ns + NS - 1) / NS, &grid)) != QGX_OK) return rc;
+  k<<<grid, NT, smem, st>>>(table, n, mp, op, spins, ns, eloc, table_floats(n, mp));
+  return launch_status();
+}
+
 template <int JT>
 int launch_eloc(const float* table, int n, int mp, const qgx_operator_t& op, const uint32_t* spins, int64_t ns,
                 double* eloc, cudaStream_t st) {
   constexpr int NT = threads_for<JT>();
+  // two samples per warp where one each would leave samples over (one CTA per SM), up to 512 hidden
+  // units (registers)
+  constexpr int NS = JT <= 4 ? 2 : 1;
+  const bool two = ns > (int64_t)device_sm_count() * (NT / 32);
   size_t smem;
-  int grid, rc;
-  if (fits_smem(NT, table_floats(n, mp), 32, &smem)) {
-    auto k = eloc_kernel<JT, true, NT>;
-    if ((rc = configure(k, NT, smem, ns, &grid)) != QGX_OK) return rc;
-    k<<<grid, NT, smem, st>>>(table, n, mp, op, spins, ns, eloc, table_floats(n, mp));
-  } else {
-    auto k = eloc_kernel<JT, false, NT>;
-    if ((rc = configure(k, NT, smem, ns, &grid)) != QGX_OK) return rc;
-    k<<<grid, NT, smem, st>>>(table, n, mp, op, spins, ns, eloc, table_floats(n, mp));
-  }
-  return launch_status();
+  if (fits_smem(NT, table_floats(n, mp), 32, &smem))
+    return two ? launch_eloc_v<JT, true, NS>(table, n, mp, op, spins, ns, eloc, smem, st)
+               : launch_eloc_v<JT, true, 1>(table, n, mp, op, spins, ns, eloc, smem, st);
+  return two ? launch_eloc_v<JT, false, NS>(table, n, mp, op, spins, ns, eloc, smem, st)
+             : launch_eloc_v<JT, false, 1>(table, n, mp, op, spins, ns, eloc, smem, st);
 }
 
 constexpr int kFwdThreads = 256;
