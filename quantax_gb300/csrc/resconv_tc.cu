@@ -147,20 +147,77 @@ __device__ inline void tmem_ld_16cols(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// GELU of a value that is next rounded to the operand type: BF16 keeps 8 bits, below the
-// error of the hardware tanh (about 2^-11); TF32 uses the exponential form
-__device__ inline float gelu_tanh_hw(float x) {
-  const float k0 = 0.7978845608028654f;
-  const float u = k0 * fmaf(0.044715f * x, x * x, x);
+// Pairs of floats in one instruction, each rounded as the scalar operation: the epilogues take most
+// of a CTA's issue slots, and with these 16384 BF16 forwards at L = 10, 8 blocks, 16 channels take
+// 0.75 ms (0.82 with scalar operations), TF32 ones 1.62 (1.66). Splitting the wait, so that half the
+// rows' epilogue runs beside the other tiles' MMAs of its own CTA, was slower (0.91): the SM's other
+// CTAs fill that time already.
+__device__ inline float2 add_pair(float2 a, float2 b) {
+  float2 c;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "add.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(c.x), "=f"(c.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return c;
+}
+__device__ inline float2 mul_pair(float2 a, float2 b) {
+  float2 c;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(c.x), "=f"(c.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return c;
+}
+__device__ inline float2 fma_pair(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ inline float2 both(float a) { return make_float2(a, a); }
+
+__device__ inline float tanh_hw(float x) {
   float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
-  const float h = 0.5f * x;
-  return fmaf(h, t, h);
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(x));
+  return t;
 }
 
+// GELU of values that are next rounded to the operand type: BF16 keeps 8 bits, below the
+// error of the hardware tanh (about 2^-11); TF32 uses the exponential form
 template <int KIND>
-__device__ inline float gelu_op(float x) {
-  return KIND == 1 ? gelu_tanh_hw(x) : gelu_fast(x);
+__device__ inline float2 gelu_op(float2 x) {
+  if (KIND == 0) return make_float2(gelu_fast(x.x), gelu_fast(x.y));
+  const float2 u = mul_pair(both(0.7978845608028654f), fma_pair(mul_pair(both(0.044715f), x), mul_pair(x, x), x));
+  const float2 h = mul_pair(both(0.5f), x);
+  return fma_pair(h, make_float2(tanh_hw(u.x), tanh_hw(u.y)), h);
+}
+
+// v = gelu(v + bias) of the 16 channels of a row
+template <int KIND>
+__device__ inline void gelu_row(float (&v)[16], const float* bias) {
+#pragma unroll
+  for (int c = 0; c < 16; c += 2) {
+    const float2 y = gelu_op<KIND>(add_pair(make_float2(v[c], v[c + 1]), *reinterpret_cast<const float2*>(bias + c)));
+    v[c] = y.x;
+    v[c + 1] = y.y;
+  }
+}
+
+// x += v + bias, v = gelu(x scale)
+template <int KIND>
+__device__ inline void residual_row(float (&x)[16], float (&v)[16], const float* bias, float scale) {
+#pragma unroll
+  for (int c = 0; c < 16; c += 2) {
+    const float2 b = *reinterpret_cast<const float2*>(bias + c);
+    const float2 s = add_pair(make_float2(x[c], x[c + 1]), add_pair(make_float2(v[c], v[c + 1]), b));
+    const float2 y = gelu_op<KIND>(mul_pair(s, both(scale)));
+    x[c] = s.x;
+    x[c + 1] = s.y;
+    v[c] = y.x;
+    v[c + 1] = y.y;
+  }
 }
 
 // The padded row of a thread's tile row: sample slot a, grid position (py, px); interior
@@ -372,8 +429,7 @@ struct TcForward {
           tmem_ld_16cols(tmem + tmem_lane + (uint32_t)(16 * j), v);
           const RowPos rp = unpack_pos(pos[k]);
           if (!rp.live) continue;
-#pragma unroll
-          for (int c = 0; c < 16; ++c) v[c] = gelu_op<KIND>(v[c] + bias[c]);
+          gelu_row<KIND>(v, bias);
           put_row<KIND>(Q, sh, rp, v);
         }
       }
@@ -390,11 +446,7 @@ struct TcForward {
           tmem_ld_16cols(tmem + tmem_lane + (uint32_t)(16 * j), v);
           const RowPos rp = unpack_pos(pos[k]);
           if (!rp.live) continue;
-#pragma unroll
-          for (int c = 0; c < 16; ++c) {
-            x[k][c] += v[c] + bias[c];
-            v[c] = gelu_op<KIND>(x[k][c] * scale);
-          }
+          residual_row<KIND>(x[k], v, bias, scale);
           if (b + 1 < sh.B) put_row<KIND>(P, sh, rp, v);
         }
       }
@@ -468,7 +520,7 @@ __global__ void __launch_bounds__(128 * WG, MINB)
 }
 
 // ---- warp-specialised forward (BF16, QGX_CONV_GROUPED) --------------------------------
-// Measured on GB300 to be slower than TcForward's three CTAs per SM (1.13 against 0.82 ms for
+// Measured on GB300 to be slower than TcForward's three CTAs per SM (1.04 against 0.75 ms for
 // 16384 forwards at L = 10, 8 blocks, 16 channels): a single
 // issuing thread gets about 115 clocks per N = 16 MMA, where three CTAs issuing side by side get
 // about 47 between them. It runs on request, and its bit-identical results check TcForward.
@@ -722,15 +774,10 @@ __global__ void __launch_bounds__(WsCfg<G, WG, RPT>::kThreads, 1)
           const RowPos rp = unpack_pos(pos[k]);
           if (!rp.live) continue;
           if ((l & 1) == 0) {  // conv1: Q = gelu(conv(P) + b1)
-#pragma unroll
-            for (int c = 0; c < 16; ++c) v[c] = gelu_op<1>(v[c] + bias[c]);
+            gelu_row<1>(v, bias);
             put_row<1>(Q, sh, rp, v);
           } else {  // conv2: x += conv(Q) + b2; the next block's P = gelu(x / sqrt(b + 2))
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-              x[k][c] += v[c] + bias[c];
-              v[c] = gelu_op<1>(x[k][c] * scale);
-            }
+            residual_row<1>(x[k], v, bias, scale);
             if (b + 1 < sh.B) put_row<1>(P, sh, rp, v);
           }
         }
