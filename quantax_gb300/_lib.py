@@ -263,8 +263,11 @@ def ptr(t: torch.Tensor | None):
 
 
 def stream_ptr(stream: torch.cuda.Stream | None = None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    """The stream's handle; by default the current one's, read without building a torch Stream (every
+    launch asks for it: 0.4 us of host time, 3.0 through torch.cuda.current_stream())."""
+    if stream is None:
+        return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return C.c_void_p(stream.cuda_stream)
 
 
 def require_cuda():
