@@ -91,9 +91,16 @@ __device__ inline void record_info(int* info, int64_t order) {
 
 __device__ inline double quiet_nan() { return __longlong_as_double(0x7FF8000000000000LL); }
 
+// How far the chain kernels of a factorisation have come: column groups published and CTAs started
+struct ChainState {
+  int groups;
+  unsigned tickets;
+};
+
 __global__ void diag_bound_kernel(const double* __restrict__ A, int64_t lda, int64_t n, RowBound bound,
-                                  int* __restrict__ info) {
+                                  ChainState* __restrict__ chain, int* __restrict__ info) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r == 0) *chain = ChainState{0, 0u};
   if (r >= n) return;
   const double a = A[r * lda + r];
   float f = 0.0f;
@@ -114,7 +121,7 @@ struct __align__(16) BlockFactor {
 
 constexpr float kFullRow = 0.52f;  // a row's squares sum to at most 1/2 (1 + rounding of its bound)
 constexpr float kFxHigh = 4.656612873077393e-10f;  // 2^-31: the unit of Fx::h
-// Work layout of the 64-column chain, potrf_block_kernel and trsm_block_kernel: the columns go in
+// Work layout of the 64-column chain, potrf_block and trsm_block: the columns go in
 // groups of four; lanes are rows, and a warp holds its 32 rows' entries of one group's columns
 // (trsm: of two, w and w + 8). A group's owner scales its four columns one after the other in
 // registers and publishes them in shared memory; after one barrier every warp takes the group's
@@ -245,16 +252,14 @@ __device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, 
 // first pivot that is not positive makes the remaining columns NaN and is recorded in *info as
 // c + k + 1 (the order of the failing leading minor, as LAPACK and cuSOLVER report it). Eight warps
 // hold rows 0 .. 31, one column group each, and eight rows 32 .. 63, two groups each; the lower
-// rows follow the upper ones by one group. The chain of 64 pivots bounds the kernel (one CTA), so
+// rows follow the upper ones by one group. The chain of 64 pivots bounds it (one CTA), so
 // the lower rows' multiply-adds and the stores are kept off the sub-cores that the chain runs on.
 // Measured: 30 us a block (62 us in FP64), about 780 clocks a column, of which the inverse square
-// root and the scaling take 500. With this kernel and the next the factorisation takes 0.99 ms at
-// n = 1024 (1.60 with FP64 blocks) and 4.4 at 4096 (7.4).
-__global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
-                                                                    int nb, RowBound bound,
-                                                                    BlockFactor* __restrict__ out,
-                                                                    int* __restrict__ info) {
-  __shared__ PotrfShared sh;
+// root and the scaling take 500. Complete groups are published in `out` for the triangular solve:
+// *groups becomes groups0 + g + 1 once group g can be read.
+__device__ inline void potrf_block(PotrfShared& sh, double* __restrict__ A, int64_t lda, int64_t c, int nb,
+                                   RowBound bound, BlockFactor* __restrict__ out, int* __restrict__ groups, int groups0,
+                                   int* __restrict__ info) {
   const int t = threadIdx.x, w = t >> 5, lane = t & 31;
   if (t < kBlk) {
     sh.e[t] = t < nb ? row_exponent(bound, c + t) : 0;
@@ -283,11 +288,10 @@ __global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __re
     s1[q] = i == j && i >= nb ? 1LL << 60 : fx_from_double(a, sh.e[i] + sh.e[j], 62);
   }
   __syncthreads();
-  // column k of 32 rows (of half h) to the matrix and to the triangular solve's copy
+  // column k of 32 rows (of half h) to the matrix
   auto store_column = [&](int k, int h) {
     const int r = 32 * h + lane;
     const Fx x = sh.l[k][r];
-    out->l[k][r] = x;
     if (r >= nb || r < k) return;
     double v;
     if (k >= sh.kfail)
@@ -297,11 +301,24 @@ __global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __re
     else
       v = fx_to_double(fx_join(x), sh.e[r] - kFxBits);
     A[(c + r) * lda + c + k] = v;
-    if (r == k) out->piv[k] = sh.piv[k];
   };
   auto store_group = [&](int g, int h) {
 #pragma unroll 1
     for (int e = 0; e < 4; ++e) store_column(4 * g + e, h);
+  };
+  // group g, complete in both halves, to the triangular solve (one warp)
+  auto publish = [&](int g) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int k = 4 * g + e;
+      if (g < 8) out->l[k][lane] = sh.l[k][lane];
+      out->l[k][32 + lane] = sh.l[k][32 + lane];
+    }
+    if (lane < 4) out->piv[4 * g + lane] = sh.piv[4 * g + lane];
+    __threadfence();
+    __syncwarp();
+    if (lane == 0)
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(groups), "r"(groups0 + g + 1) : "memory");
   };
 #pragma unroll 1
   for (int step = 0; step < 9; ++step) {
@@ -318,6 +335,7 @@ __global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __re
       }
       if (lower && g > 0) apply_group(&sh.l[k0][i], kPotrfLd, &sh.l[k0][32 + 4 * g0], kPotrfLd, s1 + 4, s2 + 4);
     }
+    if (!lower && g0 == step - 2) publish(g0);
     __syncthreads();
   }
 #pragma unroll 1
@@ -334,9 +352,12 @@ __global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __re
       store_group(g0, 1);
     } else if (g > 8 && g0 == ((g - 6) & 7)) {
       store_group(g - 1, 1);
+    } else if (g0 == ((g - 5) & 7)) {
+      publish(g - 1);
     }
     __syncthreads();
   }
+  if (!lower && g0 == 4) publish(15);
   if (!lower && g0 < 4) store_column(60 + g0, 1);
   if (t == 0 && sh.kfail < nb) record_info(info, c + sh.kfail + 1);
 }
@@ -361,32 +382,39 @@ __device__ inline void store_digits(uint8_t* S, int kblocks, int64_t r, int k, i
   }
 }
 
-// rows [r0, n) of the 64 columns at c: x L_cc^T = a with L_cc the factored diagonal block, in
-// place, and, for the update of the panel's later columns, the rows' digit slices S (slice row r -
-// r0) with exponents ex (S may be NULL). 32 rows per CTA. Bound by the integer pipe at
-// many rows (2016 multiply-adds of three instructions per row), by the chain of 64 scalings at
-// few: 25 us for 8000 rows (56 us in FP64). A row whose squares exceed its bound cannot be completed to a positive definite matrix:
-// its order is recorded and it becomes NaN.
-constexpr int kTrsmThreads = 256, kTrsmWarps = kTrsmThreads / 32;
-constexpr int kTrsmRows = 32;
+// Rows first .. first + 32 TILES - 1 of the 64 columns at c: x L_cc^T = a with L_cc the diagonal
+// block's factor, in place, and, for the update of the panel's later columns, the rows' digit slices S
+// (slice row r - r0) with exponents ex (S may be NULL). Eight warps per tile of 32 rows. Bound by the
+// integer pipe at many rows (2016 multiply-adds of three instructions per row), by the chain of 64
+// scalings at few. A row whose squares exceed its bound cannot be completed to a positive definite
+// matrix: its order is recorded and it becomes NaN. FOLLOW: the factorisation may still run; a warp
+// more copies its column groups to shared memory as they are published (*groups reaches groups0 + g +
+// 1), and the solve goes on with each as it comes. Else the whole factor is there.
+constexpr int kTileWarps = 8, kTileRows = 32;
+struct TrsmTile {
+  union {
+    double a[kTileRows][kBlk + 1];  // the rows as read
+    Fx x[kBlk][kTileRows + 1];      // the solution, [column][row]
+  };
+  float squares[kTileRows];
+  int bad[kTileRows], nan_row[kTileRows], er[kTileRows];
+};
+template <int TILES>
 struct TrsmShared {
   BlockFactor f;
-  union {
-    double a[kTrsmRows][kBlk + 1];  // the rows as read
-    Fx x[kBlk][kTrsmRows + 1];      // the solution, [column][row]
-  };
-  float squares[kTrsmRows];
-  int bad[kTrsmRows], nan_row[kTrsmRows];
-  int e[kBlk], er[kTrsmRows];
+  TrsmTile tile[TILES];
+  int e[kBlk];
+  uint64_t full[kBlk / 4];  // FOLLOW: column group copied
+  int fail;                 // a wait ran out
 };
 
-__device__ inline void trsm_group(TrsmShared& sh, int k0, int lane, int64_t* s1, int64_t* s2) {
+__device__ inline void trsm_group(const BlockFactor& f, TrsmTile& sh, int k0, int lane, int64_t* s1, int64_t* s2) {
   float squares = sh.squares[lane];
   bool bad = sh.bad[lane] != 0;
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int k = k0 + e;
-    const FxPivot piv = sh.f.piv[k];
+    const FxPivot piv = f.piv[k];
     const bool in_range = fx_in_range(s1[e], piv.t);
     Fx x = fx_split(fx_scale(s1[e], s2[e], piv, in_range));
     const float xv = (float)x.h * kFxHigh;
@@ -397,79 +425,133 @@ __device__ inline void trsm_group(TrsmShared& sh, int k0, int lane, int64_t* s1,
     x.h = -x.h;
     x.l = -x.l;
 #pragma unroll
-    for (int f = e + 1; f < 4; ++f) fx_mad(s1[f], s2[f], x, sh.f.l[k][k0 + f]);
+    for (int q = e + 1; q < 4; ++q) fx_mad(s1[q], s2[q], x, f.l[k][k0 + q]);
   }
   sh.squares[lane] = squares;
   if (bad) sh.bad[lane] = 1;
 }
 
-__global__ void __launch_bounds__(kTrsmThreads) trsm_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
-                                                                  int64_t r0, int64_t n, RowBound bound,
-                                                                  const BlockFactor* __restrict__ factor,
-                                                                  uint8_t* __restrict__ S, int* __restrict__ ex,
-                                                                  int* __restrict__ info) {
-  extern __shared__ uint8_t smem_raw[];
-  TrsmShared& sh = *reinterpret_cast<TrsmShared*>(smem_raw);
-  static_assert(sizeof(BlockFactor) % 16 == 0, "copied in 16-byte words");
-  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-  const int64_t first = r0 + (int64_t)blockIdx.x * kTrsmRows;
+template <int TILES, bool FOLLOW>
+__device__ inline void trsm_block(TrsmShared<TILES>& sh, double* __restrict__ A, int64_t lda, int64_t c, int64_t r0,
+                                  int64_t first, int64_t n, RowBound bound, const BlockFactor* __restrict__ factor,
+                                  const int* __restrict__ groups, int groups0, uint8_t* __restrict__ S,
+                                  int* __restrict__ ex, int* __restrict__ info, int32_t* __restrict__ status) {
+  constexpr int kSolvers = 32 * kTileWarps * TILES;  // threads
+  const int t = threadIdx.x, lane = t & 31;
+  if (t >= kSolvers + (FOLLOW ? 32 : 0)) return;
+  static_assert(sizeof(BlockFactor) % 16 == 0 && sizeof(FxPivot) == 16 && sizeof(Fx) == 8, "copied in 16-byte words");
+  if (!FOLLOW) {
 #pragma unroll
-  for (int e = t; e < (int)(sizeof(BlockFactor) / 16); e += kTrsmThreads)
-    reinterpret_cast<int4*>(&sh.f)[e] = reinterpret_cast<const int4*>(factor)[e];
-  if (t < kBlk) sh.e[t] = row_exponent(bound, c + t);
-  if (t < kTrsmRows) {
-    sh.er[t] = first + t < n ? row_exponent(bound, first + t) : 0;
-    sh.squares[t] = 0.0f;
-    sh.bad[t] = 0;
-    sh.nan_row[t] = 0;
+    for (int e = t; e < (int)(sizeof(BlockFactor) / 16); e += kSolvers)
+      reinterpret_cast<int4*>(&sh.f)[e] = reinterpret_cast<const int4*>(factor)[e];
   }
+  if (t == 0) {
+    if (FOLLOW)
+      for (int g = 0; g < kBlk / 4; ++g) mbar_init(&sh.full[g], 1);
+    sh.fail = 0;
+  }
+  if (t < kBlk) sh.e[t] = row_exponent(bound, c + t);
+  if (t < TILES * kTileRows) {
+    TrsmTile& tl = sh.tile[t / kTileRows];
+    const int r = t % kTileRows;
+    tl.er[r] = first + t < n ? row_exponent(bound, first + t) : 0;
+    tl.squares[r] = 0.0f;
+    tl.bad[r] = 0;
+    tl.nan_row[r] = 0;
+  }
+  if (t < kSolvers) {
 #pragma unroll
-  for (int e = t; e < kTrsmRows * kBlk; e += kTrsmThreads) {
-    const int r = e >> 6, j = e & 63;
-    sh.a[r][j] = first + r < n ? A[(first + r) * lda + c + j] : 0.0;  // rows past the matrix solve zeros
+    for (int e = t; e < TILES * kTileRows * kBlk; e += kSolvers) {
+      const int r = e >> 6, j = e & 63;
+      // rows past the matrix solve zeros
+      sh.tile[r / kTileRows].a[r % kTileRows][j] = first + r < n ? A[(first + r) * lda + c + j] : 0.0;
+    }
   }
   __syncthreads();
+  if (FOLLOW && t >= kSolvers) {  // the copying warp
+    int seen = groups0;
+    bool ok = true;
+    for (int g = 0; g < kBlk / 4; ++g) {
+      const uint64_t t0 = global_timer();
+      while (ok && seen - groups0 <= g) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(groups) : "memory");
+        if (seen - groups0 <= g && global_timer() - t0 > kWaitLimitNs) ok = false;
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        sh.fail = 1;  // the rows become NaN; the missing pivots count as failed
+        if (lane < 4) sh.f.piv[4 * g + lane] = FxPivot{0, 0};
+      } else {
+        const int4* src = reinterpret_cast<const int4*>(&factor->l[4 * g][0]);
+        int4* dst = reinterpret_cast<int4*>(&sh.f.l[4 * g][0]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[lane + 32 * q] = __ldcg(src + lane + 32 * q);
+        if (lane < 4)
+          reinterpret_cast<int4*>(sh.f.piv)[4 * g + lane] = __ldcg(reinterpret_cast<const int4*>(factor->piv) + 4 * g + lane);
+      }
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sh.full[g])) : "memory");
+    }
+    return;
+  }
+  const int tile = t / (32 * kTileWarps), w = (t >> 5) % kTileWarps;
+  TrsmTile& tl = sh.tile[tile];
+  auto tile_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + tile), "r"(32 * kTileWarps) : "memory"); };
+  auto wait_group = [&](int g) {
+    if (FOLLOW && !mbar_wait(&sh.full[g], 0)) sh.fail = 1;
+  };
   int64_t s1[8], s2[8];  // columns 4 w .. 4 w + 3 and 32 + 4 w ..
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int j = 4 * w + (q & 3) + (q >> 2) * 32;
-    const double a = sh.a[lane][j];
-    if (!dbl_finite(a)) sh.nan_row[lane] = 1;
-    s1[q] = fx_from_double(a, sh.er[lane] + sh.e[j], 62);
+    const double a = tl.a[lane][j];
+    if (!dbl_finite(a)) tl.nan_row[lane] = 1;
+    s1[q] = fx_from_double(a, tl.er[lane] + sh.e[j], 62);
     s2[q] = 0;
   }
-  __syncthreads();
+  tile_sync();
 #pragma unroll 1
   for (int g = 0; g < 8; ++g) {
     const int k0 = 4 * (g - 1);
+    if (g > 0) wait_group(g - 1);
     if (w >= g) {
-      if (g > 0) apply_group(&sh.x[k0][lane], kTrsmRows + 1, &sh.f.l[k0][4 * w], kBlk, s1, s2);
-      if (w == g) trsm_group(sh, 4 * g, lane, s1, s2);
+      if (g > 0) apply_group(&tl.x[k0][lane], kTileRows + 1, &sh.f.l[k0][4 * w], kBlk, s1, s2);
+      if (w == g) {
+        wait_group(g);
+        trsm_group(sh.f, tl, 4 * g, lane, s1, s2);
+      }
     }
     // the owner publishes before it goes on to its second group
-    if (w == g) __syncthreads();
-    if (g > 0) apply_group(&sh.x[k0][lane], kTrsmRows + 1, &sh.f.l[k0][32 + 4 * w], kBlk, s1 + 4, s2 + 4);
-    if (w != g) __syncthreads();
+    if (w == g) tile_sync();
+    if (g > 0) apply_group(&tl.x[k0][lane], kTileRows + 1, &sh.f.l[k0][32 + 4 * w], kBlk, s1 + 4, s2 + 4);
+    if (w != g) tile_sync();
   }
 #pragma unroll 1
   for (int g = 8; g < 16; ++g) {
     const int k0 = 4 * (g - 1);
+    wait_group(g - 1);
     if (w >= g - 8) {
-      apply_group(&sh.x[k0][lane], kTrsmRows + 1, &sh.f.l[k0][32 + 4 * w], kBlk, s1 + 4, s2 + 4);
-      if (w == g - 8) trsm_group(sh, 4 * g, lane, s1 + 4, s2 + 4);
+      apply_group(&tl.x[k0][lane], kTileRows + 1, &sh.f.l[k0][32 + 4 * w], kBlk, s1 + 4, s2 + 4);
+      if (w == g - 8) {
+        wait_group(g);
+        trsm_group(sh.f, tl, 4 * g, lane, s1 + 4, s2 + 4);
+      }
     }
-    __syncthreads();
+    tile_sync();
   }
+  wait_group(15);
+  const bool fail = *reinterpret_cast<volatile int*>(&sh.fail) != 0;
+  if (fail && status && lane == 0) atomicExch(status, QGX_ERR_TIMEOUT);
   // four rows per warp, two neighbouring columns per lane
   const bool pivots0 = sh.f.piv[2 * lane].m != 0, pivots1 = sh.f.piv[2 * lane + 1].m != 0;
 #pragma unroll 1
-  for (int rl = w; rl < kTrsmRows; rl += kTrsmWarps) {
-    const int64_t rr = first + rl;
+  for (int rl = w; rl < kTileRows; rl += kTileWarps) {
+    const int64_t rr = first + tile * kTileRows + rl;
     if (rr >= n) break;
-    const bool bad = sh.bad[rl] != 0, nans = bad || sh.nan_row[rl] != 0;
-    const int e = sh.er[rl];
+    const bool bad = tl.bad[rl] != 0, nans = bad || fail || tl.nan_row[rl] != 0;
+    const int e = tl.er[rl];
     if (bad && lane == 0) record_info(info, rr + 1);
-    const int64_t X0 = fx_join(sh.x[2 * lane][rl]), X1 = fx_join(sh.x[2 * lane + 1][rl]);
+    const int64_t X0 = fx_join(tl.x[2 * lane][rl]), X1 = fx_join(tl.x[2 * lane + 1][rl]);
     double* out = A + rr * lda + c + 2 * lane;
     out[0] = nans || !pivots0 ? quiet_nan() : fx_to_double(X0, e - kFxBits);
     out[1] = nans || !pivots1 ? quiet_nan() : fx_to_double(X1, e - kFxBits);
@@ -484,6 +566,63 @@ __global__ void __launch_bounds__(kTrsmThreads) trsm_block_kernel(double* __rest
     if (lane == 0) ex[sr] = bits == 0 ? 0 : e + bits - kFxBits;
     store_digits(S, kBlk / kOzKB, sr, 2 * lane, F0, F1);
   }
+}
+
+template <int TILES>
+union ChainShared {
+  PotrfShared potrf;
+  TrsmShared<TILES> trsm;
+};
+constexpr int chain_threads(int tiles) { return std::max(kPotrfThreads, 32 * (kTileWarps * tiles + 1)); }
+
+// One 64-column block of the panel chain in one launch: the diagonal block's factorisation (role 0) and
+// the triangular solve of the rows below (32 TILES rows per further role), which follows it a few column
+// groups behind and ends a few microseconds after it. A CTA's role is the order in which the CTAs
+// start: the factorisation is running before any CTA waits for it. The waiting CTAs keep their SMs from
+// the trailing update that runs beside, so this is for rows that leave it some; one tile per CTA, with
+// no other tile's integer work beside the chain, where there are few. About 50 us a block with the
+// update of the next columns (62 as two launches): n = 1056: 1.06 -> 0.87 ms, 4096: 4.36 -> 3.63, 8192:
+// 11.5 -> 10.5.
+template <int TILES>
+__global__ void __launch_bounds__(chain_threads(TILES), 1)
+    chain_block_kernel(double* __restrict__ A, int64_t lda, int64_t c, int nb, int64_t n, RowBound bound,
+                       BlockFactor* __restrict__ factor, uint8_t* __restrict__ S, int* __restrict__ ex,
+                       ChainState* __restrict__ chain, int groups0, unsigned tickets0, int* __restrict__ info,
+                       int32_t* __restrict__ status) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  ChainShared<TILES>& sh = *reinterpret_cast<ChainShared<TILES>*>(smem_raw);
+  __shared__ unsigned role_slot;
+  if (threadIdx.x == 0) role_slot = atomicAdd(&chain->tickets, 1u) - tickets0;
+  __syncthreads();
+  const unsigned role = role_slot;
+  if (role == 0) {
+    if (threadIdx.x < kPotrfThreads) potrf_block(sh.potrf, A, lda, c, nb, bound, factor, &chain->groups, groups0, info);
+  } else {
+    const int64_t r0 = c + kBlk, first = r0 + (int64_t)(role - 1) * TILES * kTileRows;
+    trsm_block<TILES, true>(sh.trsm, A, lda, c, r0, first, n, bound, factor, &chain->groups, groups0, S, ex, info,
+                            status);
+  }
+}
+
+// the same as two launches
+__global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
+                                                                    int nb, RowBound bound,
+                                                                    BlockFactor* __restrict__ factor,
+                                                                    ChainState* __restrict__ chain, int groups0,
+                                                                    int* __restrict__ info) {
+  __shared__ PotrfShared sh;
+  potrf_block(sh, A, lda, c, nb, bound, factor, &chain->groups, groups0, info);
+}
+
+__global__ void __launch_bounds__(32 * kTileWarps) trsm_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
+                                                                     int64_t n, RowBound bound,
+                                                                     const BlockFactor* __restrict__ factor,
+                                                                     uint8_t* __restrict__ S, int* __restrict__ ex,
+                                                                     int* __restrict__ info) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const int64_t r0 = c + kBlk, first = r0 + (int64_t)blockIdx.x * kTileRows;
+  trsm_block<1, false>(*reinterpret_cast<TrsmShared<1>*>(smem_raw), A, lda, c, r0, first, n, bound, factor, nullptr, 0, S,
+                       ex, info, nullptr);
 }
 
 // ---- digit slices ---------------------------------------------------------------------------
@@ -804,6 +943,7 @@ struct CholWs {
   uint8_t* s_block;           // digits of the 64 columns below a diagonal block
   int* e_block;               // n row exponents
   BlockFactor* factor;        // the current diagonal block's
+  ChainState* chain;
   RowBound bound;             // n row bounds
 };
 
@@ -818,7 +958,7 @@ int64_t chol_layout(int64_t n, void* base, CholWs* ws) {
   const int64_t o_sp0 = take(kSlices * nr * kPanel * 2), o_sp1 = take(kSlices * nr * kPanel * 2);
   const int64_t o_ep0 = take(n * 4), o_ep1 = take(n * 4);
   const int64_t o_sb = take(kSlices * nr * kBlk * 2), o_eb = take(n * 4), o_bf = take(sizeof(BlockFactor));
-  const int64_t o_rf = take(n * 4), o_re = take(n * 4);
+  const int64_t o_rf = take(n * 4), o_re = take(n * 4), o_cs = take(sizeof(ChainState));
   if (base && ws) {
     char* b = static_cast<char*>(base);
     ws->s_panel[0] = reinterpret_cast<uint8_t*>(b + o_sp0);
@@ -828,6 +968,7 @@ int64_t chol_layout(int64_t n, void* base, CholWs* ws) {
     ws->s_block = reinterpret_cast<uint8_t*>(b + o_sb);
     ws->e_block = reinterpret_cast<int*>(b + o_eb);
     ws->factor = reinterpret_cast<BlockFactor*>(b + o_bf);
+    ws->chain = reinterpret_cast<ChainState*>(b + o_cs);
     ws->bound.f = reinterpret_cast<float*>(b + o_rf);
     ws->bound.E = reinterpret_cast<int*>(b + o_re);
   }
@@ -917,24 +1058,51 @@ int chol_f64(double* A, int64_t n, int64_t lda, int* info, int32_t* status, void
   if (status) QGX_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), st));
   QGX_CHECK_CUDA(cudaEventRecord(la->start, st));
   QGX_CHECK_CUDA(cudaStreamWaitEvent(aux, la->start, 0));
+  QGX_CHECK_CUDA(cudaFuncSetAttribute(chain_block_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(ChainShared<1>)));
+  QGX_CHECK_CUDA(cudaFuncSetAttribute(chain_block_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(ChainShared<2>)));
   QGX_CHECK_CUDA(cudaFuncSetAttribute(trsm_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(TrsmShared)));
-  diag_bound_kernel<<<(unsigned)((n + 255) / 256), 256, 0, aux>>>(A, lda, n, ws.bound, info);
+                                      (int)sizeof(TrsmShared<1>)));
+  diag_bound_kernel<<<(unsigned)((n + 255) / 256), 256, 0, aux>>>(A, lda, n, ws.bound, ws.chain, info);
   ++*kernels;
   int64_t k = 0;
+  unsigned tickets = 0;  // drawn by the launches so far
+  const int64_t sms = device_sm_count();
   for (int64_t c0 = 0; c0 < n; c0 += kPanel, ++k) {
     const int64_t pe = std::min<int64_t>(c0 + kPanel, n);
     if (k >= 2) QGX_CHECK_CUDA(cudaStreamWaitEvent(aux, la->rest_done[k & 1], 0));
     // the panel chain
     for (int64_t cj = c0; cj < pe; cj += kBlk) {
       const int nb = (int)std::min<int64_t>(kBlk, n - cj);
-      potrf_block_kernel<<<1, kPotrfThreads, 0, aux>>>(A, lda, cj, nb, ws.bound, ws.factor, info);
-      ++*kernels;
       const int64_t rb = cj + kBlk;  // first row below the block
-      if (rb >= n) break;
-      trsm_block_kernel<<<(unsigned)((n - rb + kTrsmRows - 1) / kTrsmRows), kTrsmThreads, sizeof(TrsmShared), aux>>>(
-          A, lda, cj, rb, n, ws.bound, ws.factor, rb < pe ? ws.s_block : nullptr, ws.e_block, info);
-      ++*kernels;
+      const int64_t rows = std::max<int64_t>(0, n - rb);
+      const int groups0 = (int)(cj / kBlk) * (kBlk / 4);
+      uint8_t* S = rb < pe ? ws.s_block : nullptr;
+      // the rows' tiles of 32 per CTA where the factorisation and the solve share a launch; 0: they do
+      // not. One on up to half of the SMs, two on up to three quarters (n = 8192: 10.5 ms; 10.6 with one
+      // on all SMs, 11.5 without), so that the trailing update keeps some (n = 16384: 50.9 ms; 51.2 with
+      // two on all SMs, 52.8 with sharing at any size, 51.4 without).
+      const int64_t tiles = (rows + kTileRows - 1) / kTileRows;
+      const int per_cta = rows == 0 ? 0 : 2 * tiles < sms ? 1 : 2 * tiles < 3 * sms ? 2 : 0;
+      if (per_cta > 0) {
+        const unsigned grid = 1 + (unsigned)((tiles + per_cta - 1) / per_cta);
+        if (per_cta == 1)
+          chain_block_kernel<1><<<grid, chain_threads(1), sizeof(ChainShared<1>), aux>>>(
+              A, lda, cj, nb, n, ws.bound, ws.factor, S, ws.e_block, ws.chain, groups0, tickets, info, status);
+        else
+          chain_block_kernel<2><<<grid, chain_threads(2), sizeof(ChainShared<2>), aux>>>(
+              A, lda, cj, nb, n, ws.bound, ws.factor, S, ws.e_block, ws.chain, groups0, tickets, info, status);
+        tickets += grid;
+        ++*kernels;
+      } else {
+        potrf_block_kernel<<<1, kPotrfThreads, 0, aux>>>(A, lda, cj, nb, ws.bound, ws.factor, ws.chain, groups0, info);
+        ++*kernels;
+        if (rb >= n) break;
+        trsm_block_kernel<<<(unsigned)tiles, 32 * kTileWarps, sizeof(TrsmShared<1>), aux>>>(A, lda, cj, n, ws.bound,
+                                                                                            ws.factor, S, ws.e_block, info);
+        ++*kernels;
+      }
       if ((rc = launch_status()) != QGX_OK) return rc;
       // the block's columns update the rest of the panel (K = 64)
       if (rb < pe && (rc = ozaki_region(A, lda, ws.s_block, ws.e_block, rb, kBlk, rb, n - rb, pe - rb, status, aux,

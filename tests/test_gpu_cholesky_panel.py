@@ -73,3 +73,19 @@ def test_nan_entry_reaches_the_factor(cuda, row, col):
     A[row, col] = A[col, row] = np.nan
     Lf, _ = factor(A)
     assert np.isnan(Lf[row, :row + 1]).any()
+
+
+def test_leading_blocks_do_not_depend_on_the_rows_below(cuda):
+    """The rows below a diagonal block decide how its factorisation and the triangular solve are
+    launched (together with one or two row tiles per CTA, or one after the other). The factor of a
+    leading submatrix is the leading part of the whole factor, bit for bit, whichever it was."""
+    n = 7700
+    g = torch.Generator(device="cuda").manual_seed(5)
+    G = torch.randn((n, 300), generator=g, device="cuda", dtype=torch.float64)
+    A = (G @ G.T / 300 + torch.eye(n, device="cuda", dtype=torch.float64)).cpu().numpy()
+    whole, info = factor(A)
+    assert info == 0
+    for m in (7297, 5000, 2500, 2496, 2433, 700):
+        part, info = factor(A[:m, :m])
+        assert info == 0
+        assert np.array_equal(np.tril(part), np.tril(whole[:m, :m]))
