@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kStatThreads) reweight_kernel(const float* __r
 constexpr int kColThreads = 256;
 constexpr int kColRows = 128;  // rows per partial-sum chunk
 
-// per column and chunk of kColRows rows: sum of O and of r O, as float-pair sums (DSum)
+// per column and chunk of kColRows rows: sum of O and, with weights, of r O, as float-pair sums (DSum)
 __global__ void col_partial_kernel(const float* __restrict__ O, int64_t ns, int64_t np, int64_t ldo,
                                    const double* __restrict__ r, double* __restrict__ part_u,
                                    double* __restrict__ part_w) {
@@ -250,7 +250,8 @@ __global__ void col_partial_kernel(const float* __restrict__ O, int64_t ns, int6
   const int64_t chunk = blockIdx.y;
   const int64_t r0 = chunk * kColRows;
   const int64_t r1 = min(ns, r0 + kColRows);
-  for (int64_t s = r0 + threadIdx.x; s < r1; s += blockDim.x) rs[s - r0] = split_double(r ? r[s] : 1.0);
+  if (r)
+    for (int64_t s = r0 + threadIdx.x; s < r1; s += blockDim.x) rs[s - r0] = split_double(r[s]);
   __syncthreads();
   const int64_t col = blockIdx.x * (int64_t)kColThreads + threadIdx.x;
   if (col >= np) return;
@@ -258,11 +259,13 @@ __global__ void col_partial_kernel(const float* __restrict__ O, int64_t ns, int6
   for (int64_t s = r0; s < r1; ++s) {
     const float v = O[s * ldo + col];
     su.add(v);
-    const float2 rv = rs[s - r0];
-    sw.add_prod(v, rv.x, rv.y);
+    if (r) {
+      const float2 rv = rs[s - r0];
+      sw.add_prod(v, rv.x, rv.y);
+    }
   }
   part_u[chunk * np + col] = su.value();
-  part_w[chunk * np + col] = sw.value();
+  if (r) part_w[chunk * np + col] = sw.value();
 }
 
 // O[s][col] <- (O[s][col] - mean[col]) sqrt(r_s / ns) in FP32: the mean enters as two floats
@@ -669,7 +672,8 @@ int qgx_center_columns(float* O, int64_t ns, int64_t np, int64_t ldo, const doub
   cudaStream_t st = as_cuda(stream);
   dim3 g1(blocks_for(np, kColThreads), (unsigned)nchunk);
   col_partial_kernel<<<g1, kColThreads, 0, st>>>(O, ns, np, ldo, r, part_u, part_w);
-  col_reduce_kernel<<<blocks_for(np, 256), 256, 0, st>>>(part_u, part_w, nchunk, np, ns, mean_u, omean, nullptr);
+  col_reduce_kernel<<<reduce_blocks(np), kRedThreads, 0, st>>>(part_u, r ? part_w : nullptr, nchunk, np, ns, mean_u, omean,
+                                                                nullptr);
   split_mean_kernel<<<blocks_for(np, 256), 256, 0, st>>>(mean_u, np, mean2);
   const bool vec = (reinterpret_cast<uintptr_t>(O) & 15) == 0 && ldo % 4 == 0;
   const unsigned grid = (unsigned)std::min<int64_t>(ns, (int64_t)device_sm_count() * 8);

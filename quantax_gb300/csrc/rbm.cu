@@ -764,6 +764,7 @@ __global__ void colsum_kernel(const float* __restrict__ tb, const uint32_t* __re
   const int64_t s1 = min(ns, s0 + kChunkRows);
   float su = 0.0f;
   double sw = 0.0;
+#pragma unroll 8
   for (int64_t s = s0; s < s1; ++s) {
     const float sj = ((spins[s * nw + (j >> 5)] >> (j & 31)) & 1u) ? 1.0f : -1.0f;
     const float ti = tb[s * mp + i];
@@ -772,7 +773,7 @@ __global__ void colsum_kernel(const float* __restrict__ tb, const uint32_t* __re
     if (r) sw += (double)v * r[s];
   }
   part_u[blockIdx.y * np + col] = (double)su;
-  part_w[blockIdx.y * np + col] = r ? sw : (double)su;
+  if (r) part_w[blockIdx.y * np + col] = sw;
 }
 
 // Row writer for O (centred = false) or Obar (centred = true): warp per sample.
@@ -1454,8 +1455,8 @@ int qgx_rbm_obar(const float* table, int32_t n, int32_t m, int32_t has_vbias, co
   if (rc != QGX_OK) return rc;
   colsum_kernel<<<dim3((unsigned)((np + 255) / 256), (unsigned)nchunk), 256, 0, st>>>(tb, spins, n, m, mp, np, ns, r,
                                                                                      part_u, part_w);
-  col_reduce_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(part_u, part_w, nchunk, np, ns, nullptr, omean,
-                                                                  mean_f);
+  col_reduce_kernel<<<reduce_blocks(np), kRedThreads, 0, st>>>(part_u, r ? part_w : nullptr, nchunk, np, ns, nullptr, omean,
+                                                                mean_f);
   if ((rc = launch_status()) != QGX_OK) return rc;
 #define CALL(JT) launch_jacobian<JT>(table, n, m, mp, has_vbias, spins, ns, Obar, ldo, true, mean_f, r, st)
   QGX_DISPATCH_JT(mp, CALL)

@@ -10,6 +10,7 @@
 #include <mutex>
 #include <vector>
 
+#include "qgx_colstats.cuh"
 #include "qgx_common.cuh"
 
 namespace qgx {
@@ -131,22 +132,27 @@ __global__ void shift_diag_kernel(double* __restrict__ T, int64_t n, int64_t ldt
 // partial[chunk, col] = sum_{rows in chunk} A[s, col] y[s] to about 48 bits (the reference
 // forms x = A^T y in float64, solver.py:58-61, 144-146), as float-pair sums (DSum) with
 // y = yh + yl. Four columns per thread, 16-byte loads; the chunk's y split once into shared
-// memory.
-__global__ void project_partial_kernel(const float* __restrict__ A, int64_t nrow, int64_t ncol, int64_t lda,
-                                       const double* __restrict__ y, double* __restrict__ part, bool vec4) {
+// memory. The rows of a chunk go to four groups of 64 threads, whose sums are added in FP64: with
+// few columns the latency of a thread's row loads is the time (4099 rows, 1056 columns: 72 us
+// with the whole chunk per thread, 33 now).
+constexpr int kProjGroups = 4, kProjQuads = 64;
+__global__ void __launch_bounds__(kProjGroups* kProjQuads)
+    project_partial_kernel(const float* __restrict__ A, int64_t nrow, int64_t ncol, int64_t lda,
+                           const double* __restrict__ y, double* __restrict__ part, bool vec4) {
   __shared__ float2 ys[kProjRows];
+  __shared__ double sums[kProjGroups][4][kProjQuads];
   const int64_t r0 = (int64_t)blockIdx.y * kProjRows;
   const int64_t r1 = min(nrow, r0 + kProjRows);
   for (int64_t s = r0 + threadIdx.x; s < r1; s += blockDim.x) {
     ys[s - r0] = split_double(y[s]);
   }
   __syncthreads();
-  const int64_t c0 = 4 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
-  if (c0 >= ncol) return;
+  const int q = threadIdx.x % kProjQuads, g = threadIdx.x / kProjQuads;
+  const int64_t c0 = 4 * (blockIdx.x * (int64_t)kProjQuads + q);
   DSum a0, a1, a2, a3;
   if (vec4 && c0 + 3 < ncol) {
-#pragma unroll 4
-    for (int64_t s = r0; s < r1; ++s) {
+#pragma unroll 8
+    for (int64_t s = r0 + g; s < r1; s += kProjGroups) {
       const float2 yv = ys[s - r0];
       const float4 v = __ldg(reinterpret_cast<const float4*>(A + s * lda + c0));
       a0.add_prod(v.x, yv.x, yv.y);
@@ -154,8 +160,8 @@ __global__ void project_partial_kernel(const float* __restrict__ A, int64_t nrow
       a2.add_prod(v.z, yv.x, yv.y);
       a3.add_prod(v.w, yv.x, yv.y);
     }
-  } else {
-    for (int64_t s = r0; s < r1; ++s) {
+  } else if (c0 < ncol) {
+    for (int64_t s = r0 + g; s < r1; s += kProjGroups) {
       const float2 yv = ys[s - r0];
       const float* row = A + s * lda;
       a0.add_prod(__ldg(row + c0), yv.x, yv.y);
@@ -164,20 +170,19 @@ __global__ void project_partial_kernel(const float* __restrict__ A, int64_t nrow
       if (c0 + 3 < ncol) a3.add_prod(__ldg(row + c0 + 3), yv.x, yv.y);
     }
   }
-  double* p = part + blockIdx.y * ncol + c0;
-  p[0] = a0.value();
-  if (c0 + 1 < ncol) p[1] = a1.value();
-  if (c0 + 2 < ncol) p[2] = a2.value();
-  if (c0 + 3 < ncol) p[3] = a3.value();
-}
-
-__global__ void sum_partials_kernel(const double* __restrict__ part, int64_t nchunk, int64_t ncol,
-                                    double* __restrict__ x) {
-  const int64_t col = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  sums[g][0][q] = a0.value();
+  sums[g][1][q] = a1.value();
+  sums[g][2][q] = a2.value();
+  sums[g][3][q] = a3.value();
+  __syncthreads();
+  // one column per thread
+  const int64_t col = blockIdx.x * (int64_t)(4 * kProjQuads) + threadIdx.x;
   if (col >= ncol) return;
-  KahanD k;
-  for (int64_t c = 0; c < nchunk; ++c) k.add(part[c * ncol + col]);
-  x[col] = k.value();
+  const int cq = threadIdx.x / 4, ce = threadIdx.x % 4;
+  double sum = sums[0][ce][cq];
+#pragma unroll
+  for (int k = 1; k < kProjGroups; ++k) sum += sums[k][ce][cq];
+  part[blockIdx.y * ncol + col] = sum;
 }
 
 // soft inverse of the eigenvalues (solver.py:95-101), single block
@@ -632,10 +637,11 @@ int project(const float* A, int64_t nrow, int64_t ncol, int64_t lda, const doubl
   if (nchunk > 65535) return QGX_ERR_UNSUPPORTED;
   const bool vec4 = ((reinterpret_cast<uintptr_t>(A) & 15) == 0) && (lda % 4 == 0);
   ++g_kernels;
-  project_partial_kernel<<<dim3((unsigned)((ncol + 1023) / 1024), (unsigned)nchunk), 256, 0, st>>>(
-      A, nrow, ncol, lda, y, part, vec4);
+  constexpr int kCols = 4 * kProjQuads;
+  project_partial_kernel<<<dim3((unsigned)((ncol + kCols - 1) / kCols), (unsigned)nchunk), kProjGroups * kProjQuads, 0,
+                           st>>>(A, nrow, ncol, lda, y, part, vec4);
   ++g_kernels;
-  sum_partials_kernel<<<(unsigned)((ncol + 255) / 256), 256, 0, st>>>(part, nchunk, ncol, x);
+  sum_partials_kernel<<<reduce_blocks(ncol), kRedThreads, 0, st>>>(part, nchunk, ncol, x);
   return launch_status();
 }
 
@@ -792,7 +798,7 @@ int solve_gram(double* T, int64_t n, const double* b, int method, double rshift,
   ++g_kernels;
   uv_partial_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)nchunk), 256, 0, st>>>(T, n, ws.v, ws.part);
   ++g_kernels;
-  sum_partials_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ws.part, nchunk, n, ws.y);
+  sum_partials_kernel<<<reduce_blocks(n), kRedThreads, 0, st>>>(ws.part, nchunk, n, ws.y);
   return launch_status();
 }
 
@@ -869,7 +875,7 @@ int qgx_sr_solve(double* S, int64_t np, const float* A, int64_t n, int64_t lda, 
     ++g_kernels;
     uv_partial_kernel<<<dim3((unsigned)((np + 255) / 256), (unsigned)vchunk), 256, 0, st>>>(S, np, ws.v, ws.part);
     ++g_kernels;
-    sum_partials_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(ws.part, vchunk, np, x);
+    sum_partials_kernel<<<reduce_blocks(np), kRedThreads, 0, st>>>(ws.part, vchunk, np, x);
     return launch_status();
   }
   // F = A^T b into ws.f, then S x = F
