@@ -86,3 +86,10 @@ def test_local_energies_with_mixed_terms(cuda, ns, L, cplx):
     want = want if cplx else want.real
     qtx.set_default_dtype(np.float64)
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("ns", [255, 256, 512, 513, 2048, 2049, 20011])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_energy_stats_one_cta_or_cluster(cuda, ns, weighted, cplx):
+    test_energy_stats_forms(cuda, ns, weighted, cplx)
