@@ -502,11 +502,12 @@ int qgx_sr_solve(double* S, int64_t np, const float* A, int64_t n, int64_t lda,
  * lower triangle (L[i][j] at A[i lda + j], i >= j); the strict upper triangle keeps the input.
  * Read as column-major, the result is the upper factor U = L^T (A = U^T U) that cuSOLVER's
  * potrs takes with CUBLAS_FILL_MODE_UPPER. 64 x 64 diagonal blocks and their triangular solves
- * run in 60-bit fixed point (each row scaled by the root of its diagonal entry); every update C -= P P^T (P a 64- or 256-column panel) runs on the tensor cores
- * as an exact product of 8 BF16 digit slices per element (row-scaled 57-bit fixed point,
- * integer accumulation exact in FP32), folded in int64 and applied in FP64.
+ * run in 60-bit fixed point (each row scaled by the root of its diagonal entry); every update
+ * C -= P P^T (P a 64- or 256-column panel) runs on the tensor cores as an exact product of 8 BF16
+ * digit slices per element (row-scaled 57-bit fixed point, integer accumulation exact in FP32),
+ * folded in int64 and applied in FP64.
  * info (device int): 0, or the order of the first leading minor that is not positive
- * definite. status (device int, may be NULL): QGX_ERR_TIMEOUT if a tensor-core wait ran out
+ * definite. status (device int, may be NULL): QGX_ERR_TIMEOUT if a wait in a kernel ran out
  * (the factor is then invalid). Workspace: qgx_cholesky_workspace_bytes(n), 256-byte
  * aligned; no counterpart in the reference beyond the factorisation it calls. */
 int64_t qgx_cholesky_workspace_bytes(int64_t n);

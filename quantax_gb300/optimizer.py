@@ -61,7 +61,7 @@ def lstsq_pinv_eig(rtol: Optional[float] = None, atol: float = 0.0, tol_snr: flo
 
 
 def auto_shift_eig(rshift: Optional[float] = None, ashift: float = 1e-4, precision: str = "fp64") -> Solver:
-    """solver.py:80-91. precision="fp64": the FP64 Cholesky of qgx_cholesky (FP64 diagonal
+    """solver.py:80-91. precision="fp64": the FP64 Cholesky of qgx_cholesky (fixed-point diagonal
     blocks, exact tensor-core trailing updates); "fp64_lib": cuSOLVER's FP64 Cholesky;
     "mixed" factors in FP32 and refines the solution in FP64 (MinSR branch), falling back to
     the FP64 factorisation when the refinement stalls."""
