@@ -260,8 +260,43 @@ __global__ void __launch_bounds__(kTrsvThreads) trsv_upper_kernel(const float* _
 //     over the CTA): a serial substitution in one warp runs at GB300's FP64 rate of about two
 //     FMAs per clock per SM and measured slower than cuSOLVER's Xpotrs. On an ill-conditioned
 //     shifted Gram (condition number 1e10) the residual equals the substitution's.
+// A block's 64 values are their own signal: the published array starts as a NaN that arithmetic does
+// not produce (all bits set), and a waiting warp polls the values themselves. That takes one pass
+// through L2 per block of the chain where values, fence, flag and the values again took two: 3.4 us
+// a block, 4.4 before (n = 8192: 441 us each way, 570 before).
 constexpr int kNB64 = 64;
 constexpr int kT64 = 256;  // 8 warps
+constexpr unsigned long long kUnpublished = ~0ull;
+
+__device__ inline unsigned long long peek(const double* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// the published values at p0 and p1, waiting until every lane of the warp has its own; NaN and the
+// error word when the wait runs out
+__device__ inline void wait_values(const double* p0, const double* p1, double* v0, double* v1, int* err) {
+  unsigned long long a = peek(p0), b = peek(p1);
+  if (__any_sync(0xffffffffu, a == kUnpublished || b == kUnpublished)) {
+    const unsigned long long t0 = gtimer();
+    bool late = false;
+    do {
+      if (a == kUnpublished) a = peek(p0);
+      if (b == kUnpublished) b = peek(p1);
+      late = gtimer() - t0 > kFlagWaitNs;
+    } while (__any_sync(0xffffffffu, (a == kUnpublished || b == kUnpublished) && !late));
+    if (a == kUnpublished || b == kUnpublished) atomicExch(err, 1);
+  }
+  *v0 = __longlong_as_double((long long)a);
+  *v1 = __longlong_as_double((long long)b);
+}
+
+__device__ inline void publish_value(double* p, double v) {
+  unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  if (u == kUnpublished) u = 0x7FF8000000000000ull;
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(u) : "memory");
+}
 constexpr int kDP64 = kNB64 + 1;
 
 __host__ __device__ inline int64_t nblocks64(int64_t n) { return (n + kNB64 - 1) / kNB64; }
@@ -371,7 +406,7 @@ __device__ inline double warp_sum8(const double (&a)[8], int lane) {
 // forward: v_b <- L_bb^-1 (v_b - sum_{k<b} L_bk v_k), blocks in ticket order
 __global__ void __launch_bounds__(kT64) trsv64_lower_kernel(const double* __restrict__ L, int64_t n,
                                                             double* __restrict__ v, const double* __restrict__ dinv,
-                                                            int* flags, int* ticket, int epoch, int* err) {
+                                                            double* pub, int* ticket, int* err) {
   __shared__ double D[kNB64][kDP64];  // L_bb^-1
   __shared__ double part[kT64 / kNB64][kNB64];
   __shared__ double acc[kNB64];
@@ -395,8 +430,8 @@ __global__ void __launch_bounds__(kT64) trsv64_lower_kernel(const double* __rest
 #pragma unroll
       for (int r = 0; r < 2; ++r) lv[q][r] = i < nb ? L[(r0 + i) * n + c0 + lane + 32 * r] : 0.0;
     }
-    warp_wait_flag(flags + k, epoch, err);
-    const double v0 = __ldcg(v + c0 + lane), v1 = __ldcg(v + c0 + lane + 32);
+    double v0, v1;
+    wait_values(pub + c0 + lane, pub + c0 + lane + 32, &v0, &v1, err);
 #pragma unroll
     for (int q = 0; q < kRowsPerWarp; ++q) a[q] = fma(lv[q][1], v1, fma(lv[q][0], v0, a[q]));
   }
@@ -419,16 +454,17 @@ __global__ void __launch_bounds__(kT64) trsv64_lower_kernel(const double* __rest
     part[g][i] = y;
   }
   __syncthreads();
-  if (t < nb) __stcg(v + r0 + t, part[0][t] + part[1][t] + part[2][t] + part[3][t]);
-  __threadfence();
-  __syncthreads();
-  if (t == 0) st_release(flags + b, epoch);
+  if (t < kNB64) {
+    const double y = part[0][t] + part[1][t] + part[2][t] + part[3][t];
+    publish_value(pub + r0 + t, y);
+    if (t < nb) v[r0 + t] = y;  // for the backward pass
+  }
 }
 
 // backward: v_b <- L_bb^-T (v_b - sum_{k>b} L_kb^T v_k), blocks in reverse ticket order
 __global__ void __launch_bounds__(kT64) trsv64_upper_kernel(const double* __restrict__ L, int64_t n,
                                                             double* __restrict__ v, const double* __restrict__ dinv,
-                                                            int* flags, int* ticket, int epoch, int* err) {
+                                                            double* pub, int* ticket, int* err) {
   __shared__ double D[kNB64][kDP64];  // L_bb^-1
   __shared__ double part[kT64 / kNB64][kNB64];
   __shared__ double acc[kNB64];
@@ -443,7 +479,6 @@ __global__ void __launch_bounds__(kT64) trsv64_upper_kernel(const double* __rest
   constexpr int kGroups64 = kT64 / kNB64;        // 4
   constexpr int kPer64 = kNB64 / kGroups64;      // 16 rows j = g + 4 jj
   for (int e = t; e < kNB64 * kNB64; e += blockDim.x) D[e / kNB64][e % kNB64] = dinv[b * kNB64 * kNB64 + e];
-  const int* bflags = flags + nbk;
   double a = 0.0;
   for (int64_t k = nbk - 1; k > b; --k) {
     const int64_t j0 = k * kNB64;
@@ -454,11 +489,14 @@ __global__ void __launch_bounds__(kT64) trsv64_upper_kernel(const double* __rest
       const int j = g + kGroups64 * jj;
       lv[jj] = (j < kn && i < nb) ? L[(j0 + j) * n + r0 + i] : 0.0;
     }
-    warp_wait_flag(bflags + k, epoch, err);
+    // lane l < 16 brings the value of the group's row l
+    const double* row = pub + j0 + g + kGroups64 * (t & (kPer64 - 1));
+    double mine, same;
+    wait_values(row, row, &mine, &same, err);
 #pragma unroll
     for (int jj = 0; jj < kPer64; ++jj) {
-      const int j = g + kGroups64 * jj;
-      if (j < kn) a = fma(lv[jj], __ldcg(v + j0 + j), a);
+      const double x = __shfl_sync(0xffffffffu, mine, jj);
+      if (g + kGroups64 * jj < kn) a = fma(lv[jj], x, a);
     }
   }
   part[g][i] = a;
@@ -477,13 +515,14 @@ __global__ void __launch_bounds__(kT64) trsv64_upper_kernel(const double* __rest
     part[g][i] = x;
   }
   __syncthreads();
-  if (t < nb) __stcg(v + r0 + t, part[0][t] + part[1][t] + part[2][t] + part[3][t]);
-  __threadfence();
-  __syncthreads();
-  if (t == 0) st_release(flags + nbk + b, epoch);
+  if (t < kNB64) {
+    const double x = part[0][t] + part[1][t] + part[2][t] + part[3][t];
+    publish_value(pub + r0 + t, x);
+    if (t < nb) v[r0 + t] = x;
+  }
 }
 
-// a flag wait that ran out leaves wrong values: the result becomes NaN, which the caller's
+// a wait that ran out leaves wrong values: the result becomes NaN, which the caller's
 // finite check of the step turns into a skipped update
 __global__ void trsv64_nan_if_err_kernel(double* __restrict__ x, int64_t n, const int* __restrict__ err) {
   if (*err == 0) return;
@@ -495,7 +534,7 @@ __global__ void trsv64_nan_if_err_kernel(double* __restrict__ x, int64_t n, cons
 
 int64_t trsv64_rowmajor_workspace_bytes(int64_t n) {
   const int64_t nb = nblocks64(n);
-  return al256(nb * kNB64 * kNB64 * 8) + al256(2 * nb * 4) + al256(16);
+  return al256(nb * kNB64 * kNB64 * 8) + al256(2 * nb * kNB64 * 8) + al256(16);
 }
 
 // x <- L^-T L^-1 x for the row-major lower factor L (n x n, row stride n)
@@ -503,15 +542,16 @@ int trsv64_rowmajor_solve(const double* L, int64_t n, double* x, void* work, cud
   const int64_t nb = nblocks64(n);
   double* dinv = static_cast<double*>(work);
   char* w = static_cast<char*>(work) + al256(nb * kNB64 * kNB64 * 8);
-  int* flags = reinterpret_cast<int*>(w);
-  int* tickets = reinterpret_cast<int*>(w + al256(2 * nb * 4));
+  double* pub = reinterpret_cast<double*>(w);  // the forward pass's values, then the backward one's
+  int* tickets = reinterpret_cast<int*>(w + al256(2 * nb * kNB64 * 8));
   int* err = tickets + 2;
   const size_t dsmem = 2 * (size_t)kNB64 * kDP64 * 8;
   QGX_CHECK_CUDA(cudaFuncSetAttribute(dinv64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
-  QGX_CHECK_CUDA(cudaMemsetAsync(w, 0, al256(2 * nb * 4) + 16, st));  // flags, tickets, error word
+  QGX_CHECK_CUDA(cudaMemsetAsync(pub, 0xFF, 2 * nb * kNB64 * 8, st));  // kUnpublished
+  QGX_CHECK_CUDA(cudaMemsetAsync(tickets, 0, 16, st));                 // and the error word
   dinv64_kernel<<<(unsigned)nb, kDinvThreads, dsmem, st>>>(L, n, dinv);
-  trsv64_lower_kernel<<<(unsigned)nb, kT64, 0, st>>>(L, n, x, dinv, flags, tickets, 1, err);
-  trsv64_upper_kernel<<<(unsigned)nb, kT64, 0, st>>>(L, n, x, dinv, flags, tickets + 1, 1, err);
+  trsv64_lower_kernel<<<(unsigned)nb, kT64, 0, st>>>(L, n, x, dinv, pub, tickets, err);
+  trsv64_upper_kernel<<<(unsigned)nb, kT64, 0, st>>>(L, n, x, dinv, pub + nb * kNB64, tickets + 1, err);
   trsv64_nan_if_err_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1024), 256, 0, st>>>(x, n, err);
   return launch_status();
 }
