@@ -627,9 +627,10 @@ __global__ void __launch_bounds__(32 * kTileWarps) trsm_block_kernel(double* __r
 
 // ---- digit slices ---------------------------------------------------------------------------
 // Rows [0, m) of a 256-column panel (row r at A + (row0 + r) lda + col0): exponent e_r and the
-// 8 BF16 digit slices S, and the rows' bounds lowered by the panel's squares. One warp per row, two neighbouring columns per lane and step, integer
-// arithmetic throughout (an FP64 compare or conversion costs 64 clocks per warp): 12 us for 8000
-// rows, 49 MB read and written (61 us with FP64 arithmetic and two-byte stores).
+// 8 BF16 digit slices S, and the rows' bounds lowered by the panel's squares. One warp per row, two
+// neighbouring columns per lane and step, integer arithmetic throughout (an FP64 compare or conversion
+// costs 64 clocks per warp): 12 us for 8000 rows, 49 MB read and written (61 us with FP64 arithmetic
+// and two-byte stores).
 __global__ void slice_rows_kernel(const double* __restrict__ A, int64_t lda, int64_t row0, int64_t col0, int64_t m,
                                   uint8_t* __restrict__ S, int* __restrict__ ex, RowBound bound) {
   const int64_t r = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
