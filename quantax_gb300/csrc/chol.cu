@@ -196,14 +196,14 @@ __device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, 
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int k = k0 + e, src = k - row0;
-    Fx x;
+    int64_t X;
     bool in_range, positive;
     if (PIVOT) {
       const int64_t p1 = __shfl_sync(0xffffffffu, bad ? 0 : s1[e], src), p2 = __shfl_sync(0xffffffffu, s2[e], src);
       const FxInverse inv = fx_inverse(kfail < kBlk ? 0 : p1, p2);
       positive = inv.Y != 0;
       in_range = fx_in_range(s1[e], inv.t);
-      x = fx_split(fx_scale(s1[e], s2[e], inv, in_range));
+      X = fx_scale(s1[e], s2[e], inv, in_range);
       if (!positive) kfail = min(kfail, k);
       if (lane == 0) {
         sh.piv[k] = fx_pivot(inv);
@@ -213,8 +213,9 @@ __device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, 
       const FxPivot piv = sh.piv[k];
       positive = piv.m != 0;
       in_range = fx_in_range(s1[e], piv.t);
-      x = fx_split(fx_scale(s1[e], s2[e], piv, in_range));
+      X = fx_scale(s1[e], s2[e], piv, in_range);
     }
+    Fx x = fx_split(X);
     if (e == 0) {
 #pragma unroll
       for (int f = 1; f < 4; ++f) prev.column(f, s1, s2);
@@ -222,7 +223,7 @@ __device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, 
     const float xv = (float)x.h * kFxHigh;
     const float sq = fmaf(xv, xv, squares);
     const bool below = i > k && positive;
-    bad |= below && (!in_range || sq > kFullRow);
+    bad |= below && (!in_range || !fx_is_entry(X) || sq > kFullRow);
     if (below && !bad)
       squares = sq;
     else
@@ -416,10 +417,11 @@ __device__ inline void trsm_group(const BlockFactor& f, TrsmTile& sh, int k0, in
     const int k = k0 + e;
     const FxPivot piv = f.piv[k];
     const bool in_range = fx_in_range(s1[e], piv.t);
-    Fx x = fx_split(fx_scale(s1[e], s2[e], piv, in_range));
+    const int64_t X = fx_scale(s1[e], s2[e], piv, in_range);
+    Fx x = fx_split(X);
     const float xv = (float)x.h * kFxHigh;
     squares = fmaf(xv, xv, squares);
-    bad |= !in_range || squares > kFullRow;
+    bad |= !in_range || !fx_is_entry(X) || squares > kFullRow;
     if (bad) x = Fx{0, 0};
     sh.x[k][lane] = x;
     x.h = -x.h;

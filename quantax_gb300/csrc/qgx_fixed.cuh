@@ -179,11 +179,19 @@ __host__ __device__ inline FxPivot fx_pivot(const FxInverse& p) {
 // sqrt(v) of the pivot in units of 2^-(61 + t)
 __host__ __device__ inline int64_t fx_sqrt(uint64_t u, const FxPivot& p) { return (int64_t)fx_mulhi(u << 1, p.m); }
 
-// whether |v| 2^t is below 3/4: no row of a positive definite matrix exceeds it (|x| <= sqrt(1/2)
-// and the mantissa of 1 / sqrt(v) is at least 1)
+// whether |v| 2^t is below 3/4, so that fx_scale's products fit: every row of a positive definite
+// matrix passes (|x| <= sqrt(1/2) and the mantissa of 1 / sqrt(v) is at least 1), but so do others, whose
+// x reaches 1.5: fx_is_entry looks at the scaled value
 __host__ __device__ inline bool fx_in_range(int64_t s1, int t) {
   const int top = (int)(s1 >> 32);
   return (top < 0 ? -top : top) <= ((3 << 28) >> t);
+}
+
+// whether X, in units of 2^-60, is below 3/4 (up to 2^-28): every entry of a positive definite matrix's
+// factor is, and fx_split holds it (its high part has 32 bits: |x| < 1)
+__host__ __device__ inline bool fx_is_entry(int64_t X) {
+  const int top = (int)(X >> 32);
+  return (top < 0 ? -top : top) <= (3 << 26);
 }
 
 // x = v 2^t m 2^-62 in units of 2^-60 (0 unless in range)
