@@ -502,10 +502,14 @@ int qgx_sr_solve(double* S, int64_t np, const float* A, int64_t n, int64_t lda,
  * lower triangle (L[i][j] at A[i lda + j], i >= j); the strict upper triangle keeps the input.
  * Read as column-major, the result is the upper factor U = L^T (A = U^T U) that cuSOLVER's
  * potrs takes with CUBLAS_FILL_MODE_UPPER. 64 x 64 diagonal blocks and their triangular solves
- * run in 60-bit fixed point (each row scaled by the root of its diagonal entry); every update
- * C -= P P^T (P a 64- or 256-column panel) runs on the tensor cores as an exact product of 8 BF16
- * digit slices per element (row-scaled 57-bit fixed point, integer accumulation exact in FP32),
- * folded in int64 and applied in FP64.
+ * run in 60-bit fixed point (each row scaled by the root of its diagonal entry), or in FP64
+ * where more than a quarter of some row's and column's non-zero entries are below about 2^-10
+ * sqrt(a_ii a_jj): rows that hardly interact keep FP64's relative accuracy in every entry, otherwise
+ * an entry of L is kept to about 2^-60 sqrt(a_ii), and a pivot below about 2^-56 a_ii counts as not
+ * positive. QGX_SOLVE_SHIFT_LIB factors in FP64 throughout. Every update C -= P P^T (P a 64- or
+ * 256-column panel) runs on the tensor cores as an exact product of 8 BF16 digit slices per element
+ * (row-scaled 57-bit fixed point, integer accumulation exact in FP32), folded in int64 and applied
+ * in FP64.
  * info (device int): 0, or the order of the first leading minor that is not positive
  * definite. status (device int, may be NULL): QGX_ERR_TIMEOUT if a wait in a kernel ran out
  * (the factor is then invalid). Workspace: qgx_cholesky_workspace_bytes(n), 256-byte

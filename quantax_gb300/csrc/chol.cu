@@ -7,8 +7,8 @@
 // U = L^T with A = U^T U.
 //
 // FP64 arithmetic runs at about two FMAs per clock per SM on GB300 and every FP64 instruction
-// takes 64 clocks, so nothing here runs on the FP64 pipe but the last step of an update:
-// right-looking, 256-column panels, each factored as four 64-column blocks (potrf of the 64 x 64
+// takes 64 clocks, so nothing here runs on the FP64 pipe but the last step of an update (and the panels
+// of a matrix whose rows hardly interact, see weak_coupling_kernel): right-looking, 256-column panels, each factored as four 64-column blocks (potrf of the 64 x 64
 // diagonal block and the 64-wide triangular solve of every row below it) in 60-bit fixed point
 // on the integer pipe (qgx_fixed.cuh). Every update of the form C -= P P^T runs on the tensor cores
 // as an exact integer product (the Ozaki scheme: Ozaki, Ogita, Oishi and Rump, "Error-free
@@ -44,7 +44,7 @@ namespace qgx {
 namespace {
 
 constexpr int kPanel = 256;                     // columns of one tensor-core trailing update
-constexpr int kBlk = 64;                        // columns of one FP64 diagonal block
+constexpr int kBlk = 64;                        // columns of one diagonal block
 constexpr int kSlices = 8;                      // BF16 digits per element
 constexpr int kFixBits = 56;                    // kSlices * 7 fraction bits of the sliced rows
 constexpr int kOzM = 128, kOzN = 64, kOzKB = 32;  // tile rows, tile columns, K per stage
@@ -91,17 +91,21 @@ __device__ inline void record_info(int* info, int64_t order) {
 
 __device__ inline double quiet_nan() { return __longlong_as_double(0x7FF8000000000000LL); }
 
-// How far the chain kernels of a factorisation have come: column groups published and CTAs started
+// How far the chain kernels of a factorisation have come (column groups published, CTAs started) and
+// the arithmetic of its panel: FP64 if the tickets' top bit is set (choose_panel_kernel). A CTA has it
+// with its ticket, and a load of its own would be half a microsecond of every block.
 struct ChainState {
   int groups;
   unsigned tickets;
 };
+constexpr unsigned kPanelFp64 = 1u << 31;
 
 __global__ void diag_bound_kernel(const double* __restrict__ A, int64_t lda, int64_t n, RowBound bound,
-                                  ChainState* __restrict__ chain, int* __restrict__ info) {
+                                  ChainState* __restrict__ chain, int* __restrict__ score, int* __restrict__ info) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r == 0) *chain = ChainState{0, 0u};
   if (r >= n) return;
+  score[r] = 0;
   const double a = A[r * lda + r];
   float f = 0.0f;
   int E = 0;
@@ -111,6 +115,73 @@ __global__ void diag_bound_kernel(const double* __restrict__ A, int64_t lda, int
     record_info(info, r + 1);
   bound.f[r] = f;
   bound.E[r] = E;
+}
+
+// Which arithmetic the panel takes. Fixed point keeps an entry of L to 2^-61 of its row's scale 2^e_r,
+// FP64 to 2^-53 of itself: the first is the better where the entries of A are not far below sqrt(a_rr
+// a_kk) (the errors of FP64's sums are those of the large products), the second where rows hardly
+// interact. So the entries of A below the diagonal are counted: a weak one is not zero and below 2^-12
+// 2^(e_r + e_k) (2^-9 to 2^-11 of sqrt(a_rr a_kk)), and if of any row and its column more than a quarter
+// of the entries that are not zero are weak, the panel is factored in FP64. Random couplings of size c
+// beside the diagonal, n = 64, median relative error of an entry of L, FP64 and fixed point: 1.1e-16 and
+// 4.5e-17 at c = 2^-4, 7.9e-17 and 1.2e-16 at 2^-7 (a tenth of the entries weak), 7.7e-17 and 2.4e-16 at
+// 2^-8 (a fifth, of some row more than a quarter), 7.5e-17 and 9.7e-13 at 2^-20. Of a Gram of RBM or
+// ResConv samples 1 to 5% are weak (13% in a row of 6000 samples of 65536 parameters).
+// One pass over the lower triangle: 8 us of 0.90 ms at n = 1056, 0.1 of 10.7 ms at 8192.
+constexpr int kWeakBits = 12, kWeakTile = 64, kWeakThreads = 256;
+__global__ void __launch_bounds__(kWeakThreads)
+    weak_coupling_kernel(const double* __restrict__ A, int64_t lda, int64_t n, RowBound bound, int* __restrict__ score) {
+  __shared__ int er[kWeakTile], ec[kWeakTile], col_score[kWeakTile];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  // lower-triangular tile index -> (bi, bj), bi >= bj
+  const int64_t tile = blockIdx.x;
+  int64_t bi = (int64_t)((sqrtf(8.0f * (float)tile + 1.0f) - 1.0f) * 0.5f);
+  while ((bi + 1) * (bi + 2) / 2 <= tile) ++bi;
+  while (bi * (bi + 1) / 2 > tile) --bi;
+  const int64_t r0 = bi * kWeakTile, c0 = (tile - bi * (bi + 1) / 2) * kWeakTile;
+  constexpr int kWarps = kWeakThreads / 32, kRows = kWeakTile / kWarps;  // rows per warp
+  uint32_t hi[kRows][2];  // high words, the sign out; 1 for a value that only the low word holds
+#pragma unroll
+  for (int k = 0; k < kRows; ++k)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int64_t r = r0 + warp + k * kWarps, j = c0 + 32 * q + lane;
+      const uint64_t b = r < n && j < r ? dbl_bits(A[r * lda + j]) << 1 : 0;
+      hi[k][q] = (uint32_t)(b >> 33) | ((uint32_t)b != 0);
+    }
+  if (t < kWeakTile) {
+    er[t] = r0 + t < n ? row_exponent(bound, r0 + t) : 0;
+    ec[t] = c0 + t < n ? row_exponent(bound, c0 + t) : 0;
+    col_score[t] = 0;
+  }
+  __syncthreads();
+  int cs[2] = {};  // scores: 3 for a weak entry, -1 for another that is not zero
+#pragma unroll
+  for (int k = 0; k < kRows; ++k) {
+    const int i = warp + k * kWarps;
+    int rs = 0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      // |a| < 2^(exponent field - 1022)
+      const int s = hi[k][q] == 0 ? 0 : (int)(hi[k][q] >> 20) - 1022 <= er[i] + ec[32 * q + lane] - kWeakBits ? 3 : -1;
+      rs += s;
+      cs[q] += s;
+    }
+    rs = __reduce_add_sync(0xffffffffu, rs);
+    if (lane == 0 && rs != 0) atomicAdd(score + r0 + i, rs);
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) atomicAdd(&col_score[32 * q + lane], cs[q]);
+  __syncthreads();
+  if (t < kWeakTile && col_score[t] != 0) atomicAdd(score + c0 + t, col_score[t]);
+}
+
+constexpr int kChooseThreads = 1024;
+__global__ void __launch_bounds__(kChooseThreads) choose_panel_kernel(const int* __restrict__ score, int64_t n,
+                                                                      ChainState* __restrict__ chain) {
+  int any = 0;
+  for (int64_t r = threadIdx.x; r < n; r += kChooseThreads) any |= score[r] > 0;
+  if (__syncthreads_or(any) && threadIdx.x == 0) chain->tickets = kPanelFp64;
 }
 
 // the block's factor in fixed point, as the triangular solve reads it
@@ -174,6 +245,7 @@ struct PotrfShared {
   int e[kBlk];
   int bad[kBlk];         // row cannot belong to a positive definite matrix
   int kfail;             // first column whose pivot failed
+  double root[2];        // FP64: the pivot's square root and its inverse
 };
 
 // the warp's 32 rows (from row0) of the columns k0 .. k0 + 3, scaled and published; all updates are
@@ -249,6 +321,44 @@ __device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, 
   if (PIVOT && lane == 0) sh.kfail = kfail;
 }
 
+// The diagonal block's factorisation in FP64, for matrices whose rows hardly interact
+// (choose_panel_kernel), from sh.a: bound by FP64 instructions (64 clocks of a sub-core each). 512
+// threads as a 32 x 16 grid over the trailing block; the pivot's inverse square root scales its column.
+// *groups becomes groups0 + 16 once the block can be read from A.
+__device__ __noinline__ void potrf_block_fp64(PotrfShared& sh, double* __restrict__ A, int64_t lda, int64_t c, int nb,
+                                        int* __restrict__ groups, int groups0, int* __restrict__ info) {
+  const int t = threadIdx.x, ti = t >> 4, tj = t & 15;
+  constexpr int kRows = kPotrfThreads / 16;
+  for (int k = 0; k < nb; ++k) {
+    if (t == 0) {
+      double d = sh.a[k][k];
+      if (!(d > 0.0)) {
+        record_info(info, c + k + 1);
+        d = quiet_nan();
+      }
+      const double r = rsqrt(d);
+      sh.root[0] = d * r;  // sqrt(d)
+      sh.root[1] = r;
+    }
+    __syncthreads();
+    const double r = sh.root[1];
+    if (t == 0) sh.a[k][k] = sh.root[0];
+    for (int i = k + 1 + t; i < nb; i += kPotrfThreads) sh.a[i][k] *= r;
+    __syncthreads();
+    for (int i = k + 1 + ti; i < nb; i += kRows) {
+      const double aik = sh.a[i][k];
+      for (int j = k + 1 + tj; j <= i; j += 16) sh.a[i][j] = fma(-aik, sh.a[j][k], sh.a[i][j]);
+    }
+    __syncthreads();
+  }
+  for (int i = ti; i < nb; i += kRows)
+    for (int j = tj; j <= i; j += 16) A[(c + i) * lda + c + j] = sh.a[i][j];
+  __threadfence();
+  __syncthreads();
+  if (t == 0)
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(groups), "r"(groups0 + kBlk / 4) : "memory");
+}
+
 // Cholesky of the nb x nb (nb <= 64) diagonal block at (c, c), in place, in fixed point. The
 // first pivot that is not positive makes the remaining columns NaN and is recorded in *info as
 // c + k + 1 (the order of the failing leading minor, as LAPACK and cuSOLVER report it). Eight warps
@@ -258,7 +368,7 @@ __device__ inline void solve_group(PotrfShared& sh, int k0, int row0, int lane, 
 // Measured: 30 us a block (62 us in FP64), about 780 clocks a column, of which the inverse square
 // root and the scaling take 500. Complete groups are published in `out` for the triangular solve:
 // *groups becomes groups0 + g + 1 once group g can be read.
-__device__ inline void potrf_block(PotrfShared& sh, double* __restrict__ A, int64_t lda, int64_t c, int nb,
+__device__ inline void potrf_block(PotrfShared& sh, bool fp64, double* __restrict__ A, int64_t lda, int64_t c, int nb,
                                    RowBound bound, BlockFactor* __restrict__ out, int* __restrict__ groups, int groups0,
                                    int* __restrict__ info) {
   const int t = threadIdx.x, w = t >> 5, lane = t & 31;
@@ -274,6 +384,10 @@ __device__ inline void potrf_block(PotrfShared& sh, double* __restrict__ A, int6
     sh.a[r][j] = r < nb && j <= r ? A[(c + r) * lda + c + j] : 0.0;
   }
   __syncthreads();
+  if (fp64) {
+    potrf_block_fp64(sh, A, lda, c, nb, groups, groups0, info);
+    return;
+  }
   // warps 0, 1 (mod 4): the upper rows, on two of the SM's four sub-cores; 2, 3: the lower ones
   const bool lower = (w & 2) != 0;
   const int g0 = (w >> 2) * 2 + (w & 1), row0 = lower ? 32 : 0, i = row0 + lane;
@@ -570,10 +684,89 @@ __device__ inline void trsm_block(TrsmShared<TILES>& sh, double* __restrict__ A,
   }
 }
 
+// The same in FP64, for matrices whose rows hardly interact (choose_panel_kernel), from the diagonal
+// block in A (FOLLOW: once it is published whole). Eight lanes per row, lane l holding columns l, l + 8,
+// ..., l + 56: the owner of column k scales it and hands it to the others, which update their later
+// columns. Bound by FP64 instructions.
+struct TrsmFp64Shared {
+  double l[kBlk][kBlk + 1];
+  double rec[kBlk];  // 1 / l_kk
+  int fail;          // the wait ran out
+};
+template <int TILES, bool FOLLOW>
+__device__ inline void trsm_block_fp64(TrsmFp64Shared& sh, double* __restrict__ A, int64_t lda, int64_t c, int64_t r0,
+                                       int64_t first, int64_t n, const int* __restrict__ groups, int groups0,
+                                       uint8_t* __restrict__ S, int* __restrict__ ex, int32_t* __restrict__ status) {
+  constexpr int kSolvers = 32 * kTileWarps * TILES;  // threads, eight per row
+  const int t = threadIdx.x;
+  if (t >= kSolvers) return;
+  if (t == 0) {
+    int seen = groups0 + kBlk / 4;
+    if (FOLLOW) {
+      const uint64_t t0 = global_timer();
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(groups) : "memory");
+      } while (seen - groups0 < kBlk / 4 && global_timer() - t0 <= kWaitLimitNs);
+    }
+    sh.fail = seen - groups0 < kBlk / 4;
+    if (sh.fail && status) atomicExch(status, QGX_ERR_TIMEOUT);
+  }
+  __syncthreads();
+  for (int e = t; e < kBlk * kBlk; e += kSolvers) {
+    const int i = e / kBlk, j = e % kBlk;
+    sh.l[i][j] = j <= i ? __ldcg(A + (c + i) * lda + c + j) : 0.0;
+  }
+  __syncthreads();
+  if (t < kBlk) sh.rec[t] = 1.0 / sh.l[t][t];
+  __syncthreads();
+  const int sub = t & 7;
+  const int64_t r = first + (t >> 3);
+  const bool live = r < n;  // eight lanes share a row; those past the matrix solve zeros
+  double* row = A + (live ? r : r0) * lda + c;
+  double x[kBlk / 8];
+#pragma unroll
+  for (int q = 0; q < kBlk / 8; ++q) x[q] = live ? row[8 * q + sub] : 0.0;
+#pragma unroll
+  for (int k = 0; k < kBlk; ++k) {
+    const int qk = k >> 3;
+    double xk = 0.0;
+    if (sub == (k & 7)) {
+      x[qk] *= sh.rec[k];
+      xk = x[qk];
+    }
+    xk = __shfl_sync(0xffffffffu, xk, k & 7, 8);
+#pragma unroll
+    for (int q = 0; q < kBlk / 8; ++q)
+      if (8 * q + sub > k) x[q] = fma(-xk, sh.l[8 * q + sub][k], x[q]);
+  }
+  uint64_t mx = 0;
+#pragma unroll
+  for (int q = 0; q < kBlk / 8; ++q) {
+    if (sh.fail) x[q] = quiet_nan();
+    if (live) row[8 * q + sub] = x[q];
+    const uint64_t b = dbl_bits(x[q]) & 0x7FFFFFFFFFFFFFFFULL;
+    mx = b < 0x7FF0000000000000ULL && b > mx ? b : mx;  // NaN and infinities slice as zero
+  }
+  if (S == nullptr) return;
+  // the row's exponent and digits, as slice_rows_kernel takes them
+  int top = mx == 0 ? -1 : max((int)(mx >> 52), 1);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+  const int e = top < 0 ? 0 : top - 1022;
+  if (live && sub == 0) ex[r - r0] = e;
+#pragma unroll
+  for (int q = 0; q < kBlk / 8; ++q) {
+    const int64_t F = fx_from_double(x[q], e, kFixBits);
+    const int64_t next = __shfl_down_sync(0xffffffffu, F, 1);
+    if (live && (sub & 1) == 0) store_digits(S, kBlk / kOzKB, r - r0, 8 * q + sub, F, next);
+  }
+}
+
 template <int TILES>
 union ChainShared {
   PotrfShared potrf;
   TrsmShared<TILES> trsm;
+  TrsmFp64Shared trsm_fp64;
 };
 constexpr int chain_threads(int tiles) { return std::max(kPotrfThreads, 32 * (kTileWarps * tiles + 1)); }
 
@@ -596,11 +789,17 @@ __global__ void __launch_bounds__(chain_threads(TILES), 1)
   __shared__ unsigned role_slot;
   if (threadIdx.x == 0) role_slot = atomicAdd(&chain->tickets, 1u) - tickets0;
   __syncthreads();
-  const unsigned role = role_slot;
+  const bool fp64 = (role_slot & kPanelFp64) != 0;
+  const unsigned role = role_slot & ~kPanelFp64;
   if (role == 0) {
-    if (threadIdx.x < kPotrfThreads) potrf_block(sh.potrf, A, lda, c, nb, bound, factor, &chain->groups, groups0, info);
+    if (threadIdx.x < kPotrfThreads)
+      potrf_block(sh.potrf, fp64, A, lda, c, nb, bound, factor, &chain->groups, groups0, info);
   } else {
     const int64_t r0 = c + kBlk, first = r0 + (int64_t)(role - 1) * TILES * kTileRows;
+    if (fp64) {
+      trsm_block_fp64<TILES, true>(sh.trsm_fp64, A, lda, c, r0, first, n, &chain->groups, groups0, S, ex, status);
+      return;
+    }
     trsm_block<TILES, true>(sh.trsm, A, lda, c, r0, first, n, bound, factor, &chain->groups, groups0, S, ex, info,
                             status);
   }
@@ -613,16 +812,22 @@ __global__ void __launch_bounds__(kPotrfThreads) potrf_block_kernel(double* __re
                                                                     ChainState* __restrict__ chain, int groups0,
                                                                     int* __restrict__ info) {
   __shared__ PotrfShared sh;
-  potrf_block(sh, A, lda, c, nb, bound, factor, &chain->groups, groups0, info);
+  potrf_block(sh, (__ldcg(&chain->tickets) & kPanelFp64) != 0, A, lda, c, nb, bound, factor, &chain->groups, groups0, info);
 }
 
 __global__ void __launch_bounds__(32 * kTileWarps) trsm_block_kernel(double* __restrict__ A, int64_t lda, int64_t c,
                                                                      int64_t n, RowBound bound,
                                                                      const BlockFactor* __restrict__ factor,
+                                                                     const ChainState* __restrict__ chain,
                                                                      uint8_t* __restrict__ S, int* __restrict__ ex,
                                                                      int* __restrict__ info) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const int64_t r0 = c + kBlk, first = r0 + (int64_t)blockIdx.x * kTileRows;
+  if ((__ldcg(&chain->tickets) & kPanelFp64) != 0) {
+    trsm_block_fp64<1, false>(*reinterpret_cast<TrsmFp64Shared*>(smem_raw), A, lda, c, r0, first, n, nullptr, 0, S, ex,
+                              nullptr);
+    return;
+  }
   trsm_block<1, false>(*reinterpret_cast<TrsmShared<1>*>(smem_raw), A, lda, c, r0, first, n, bound, factor, nullptr, 0, S,
                        ex, info, nullptr);
 }
@@ -1035,13 +1240,13 @@ int look_ahead_for_current_device(LookAhead** out) {
 int64_t chol_f64_workspace_bytes(int64_t n) { return n > 0 ? chol_layout(n, nullptr, nullptr) : 0; }
 
 // A = L L^T in place (see the file comment). info: 0, or the order of the first leading minor
-// that is not positive definite. status (may be NULL): QGX_ERR_TIMEOUT if a tensor-core wait ran
-// out. Adds the number of kernels launched to *kernels.
+// that is not positive definite. status (may be NULL): QGX_ERR_TIMEOUT if a wait ran out, a tensor
+// core's or the chain's. Adds the number of kernels launched to *kernels.
 //
 // Look-ahead: panel k's trailing update is split into the next panel's 256 columns (the strip)
-// and the rest. The panel chain (FP64 diagonal blocks, triangular solves, the in-panel updates),
-// the panel's slicing and the strip run on a high-priority internal stream; the rest runs on the
-// caller's stream, so the next panel's FP64 chain overlaps the large tensor-core update. Panel
+// and the rest. The panel chain (diagonal blocks, triangular solves, the in-panel updates), the
+// panel's slicing and the strip run on a high-priority internal stream; the rest runs on the
+// caller's stream, so the next panel's chain overlaps the large tensor-core update. Panel
 // k's chain waits for the rest update of panel k - 2, and panel k's strip for the rest update of
 // panel k - 1: every update of a column block is ordered after the previous one (the strip and
 // the previous panel's rest both update the next panel's columns below its diagonal). Two slice
@@ -1067,8 +1272,13 @@ int chol_f64(double* A, int64_t n, int64_t lda, int* info, int32_t* status, void
                                       (int)sizeof(ChainShared<2>)));
   QGX_CHECK_CUDA(cudaFuncSetAttribute(trsm_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)sizeof(TrsmShared<1>)));
-  diag_bound_kernel<<<(unsigned)((n + 255) / 256), 256, 0, aux>>>(A, lda, n, ws.bound, ws.chain, info);
-  ++*kernels;
+  int* score = ws.e_panel[1];  // free until the second panel is sliced
+  diag_bound_kernel<<<(unsigned)((n + 255) / 256), 256, 0, aux>>>(A, lda, n, ws.bound, ws.chain, score, info);
+  const int64_t scans = (n + kWeakTile - 1) / kWeakTile, scan_tiles = scans * (scans + 1) / 2;
+  if (scan_tiles > 0x7fffffffLL) return QGX_ERR_UNSUPPORTED;
+  weak_coupling_kernel<<<(unsigned)scan_tiles, kWeakThreads, 0, aux>>>(A, lda, n, ws.bound, score);
+  choose_panel_kernel<<<1, kChooseThreads, 0, aux>>>(score, n, ws.chain);
+  *kernels += 3;
   int64_t k = 0;
   unsigned tickets = 0;  // drawn by the launches so far
   const int64_t sms = device_sm_count();
@@ -1102,8 +1312,8 @@ int chol_f64(double* A, int64_t n, int64_t lda, int* info, int32_t* status, void
         potrf_block_kernel<<<1, kPotrfThreads, 0, aux>>>(A, lda, cj, nb, ws.bound, ws.factor, ws.chain, groups0, info);
         ++*kernels;
         if (rb >= n) break;
-        trsm_block_kernel<<<(unsigned)tiles, 32 * kTileWarps, sizeof(TrsmShared<1>), aux>>>(A, lda, cj, n, ws.bound,
-                                                                                            ws.factor, S, ws.e_block, info);
+        trsm_block_kernel<<<(unsigned)tiles, 32 * kTileWarps, sizeof(TrsmShared<1>), aux>>>(
+            A, lda, cj, n, ws.bound, ws.factor, ws.chain, S, ws.e_block, info);
         ++*kernels;
       }
       if ((rc = launch_status()) != QGX_OK) return rc;

@@ -13,7 +13,8 @@
 // xl yl is below 2^-64; over 64 columns the sums stay below 2^63 by Cauchy-Schwarz). Against
 // FP64, whose roundings are relative to each value: x is kept to 2^-61 of 2^e_r <= 2.9
 // sqrt(a_rr), the FP64 spacing of an entry of 2^-7 sqrt(a_rr), which is the typical size in a
-// row of 16384 columns.
+// row of 16384 columns. Entries far below that are held in fewer bits than FP64 has, so matrices with
+// many of them are not factored this way (chol.cu, weak_coupling_kernel).
 #pragma once
 
 #include <stdint.h>

@@ -61,8 +61,9 @@ def lstsq_pinv_eig(rtol: Optional[float] = None, atol: float = 0.0, tol_snr: flo
 
 
 def auto_shift_eig(rshift: Optional[float] = None, ashift: float = 1e-4, precision: str = "fp64") -> Solver:
-    """solver.py:80-91. precision="fp64": the FP64 Cholesky of qgx_cholesky (fixed-point diagonal
-    blocks, exact tensor-core trailing updates); "fp64_lib": cuSOLVER's FP64 Cholesky;
+    """solver.py:80-91. precision="fp64": the FP64 Cholesky of qgx_cholesky (diagonal blocks in
+    60-bit fixed point, relative to their rows, or in FP64 where rows hardly interact; exact
+    tensor-core trailing updates); "fp64_lib": cuSOLVER's FP64 Cholesky;
     "mixed" factors in FP32 and refines the solution in FP64 (MinSR branch), falling back to
     the FP64 factorisation when the refinement stalls."""
     if precision not in ("fp64", "fp64_lib", "mixed"):
