@@ -114,7 +114,8 @@ __host__ __device__ inline int64_t fx_combine(int64_t s1, int64_t s2, int t) {
   return (int64_t)(((uint64_t)s1 << t) + (uint64_t)(s2 >> (29 - t)));
 }
 
-// floor of a b / 2^64 up to 2 units below, a < 3/4 2^64 or b < 2^63, the other below 2^63
+// floor of a b / 2^64 up to 2 units below, a and b at most 2^63, or a < 2^63 and b < 2^63 + 2^32: the two
+// cross products have to stay below 2^64 together
 __host__ __device__ inline uint64_t fx_mulhi(uint64_t a, uint64_t b) {
   const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
   const uint64_t mid = (uint64_t)ah * bl + (uint64_t)al * bh;

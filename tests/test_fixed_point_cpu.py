@@ -24,6 +24,9 @@ static int exponent(double a) {
   return ((f == 1.0 ? 1 : 0) + E + 2) >> 1;
 }
 
+extern "C" uint64_t pivot(int64_t v) { return fx_pivot(fx_inverse(v, 0)).m; }
+extern "C" uint64_t mulhi(uint64_t a, uint64_t b) { return fx_mulhi(a, b); }
+
 // n x n (n <= 64) lower factor of A (row-major, in place); the order of the first failing minor, or 0
 extern "C" int factor(double* A, int n) {
   static Fx l[64][64];  // [column][row]
@@ -79,7 +82,12 @@ def host(tmp_path_factory):
     assert gxx, "g++ builds the library's host code"
     subprocess.run([gxx, "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC", "-I", str(CSRC), "-o",
                     str(d / "host.so"), str(d / "host.cpp")], check=True)
-    return C.CDLL(str(d / "host.so"))
+    lib = C.CDLL(str(d / "host.so"))
+    lib.mulhi.restype = C.c_uint64
+    lib.mulhi.argtypes = [C.c_uint64, C.c_uint64]
+    lib.pivot.restype = C.c_uint64
+    lib.pivot.argtypes = [C.c_int64]
+    return lib
 
 
 def factor(host, A):
@@ -103,3 +111,28 @@ def test_two_by_two_matrices_are_told_apart(host):
                     if r < 1.0:
                         assert abs(L[1, 0] * L[0, 0] - a) <= 2.0 ** -51 * np.sqrt(d0 * d1)
                         assert abs(L[1] @ L[1] - d1) <= 2.0 ** -51 * d1
+
+
+def test_high_products_at_the_ends_of_their_range(host):
+    """fx_mulhi against whole products: at most 2 below the floor for factors up to 2^63, and for one
+    below 2^63 with one below 2^63 + 2^32 (the mantissa of an inverse square root may round past 2)."""
+    rng = np.random.default_rng(0)
+    ends = [0, 1, 2 ** 32 - 1, 2 ** 32, 2 ** 62, 2 ** 63 - 2 ** 32, 2 ** 63 - 1, 2 ** 63]
+    some = [int(v) for v in rng.integers(0, 2 ** 63, 2000)]
+    past = [2 ** 63 + 1, 2 ** 63 + 2 ** 31, 2 ** 63 + 2 ** 32 - 1]
+    pairs = [(a, b) for a in ends + some[:50] for b in ends + some[:50]] + list(zip(some, some[::-1]))
+    pairs += [(a, b) for a in ends[:-1] + some for b in past]
+    for a, b in pairs:
+        exact = a * b >> 64
+        for got in (host.mulhi(a, b), host.mulhi(b, a)):
+            assert exact - 2 <= got <= exact, (a, b)
+
+
+def test_every_inverse_square_root_fits_the_products(host):
+    """The factors that fx_inverse, fx_sqrt and fx_scale multiply: pivots beside the powers of two and
+    over the whole range, whose mantissas m 2^-62 of 1 / sqrt(v) lie in [1, 2] up to the estimate."""
+    rng = np.random.default_rng(1)
+    ends = [m + d for k in range(4, 62) for m in (2 ** k,) for d in (-1, 0, 1) if 16 <= m + d <= 2 ** 61]
+    for v in ends + [int(x) for x in np.exp2(rng.uniform(4, 61, 4000))]:
+        m = host.pivot(v)
+        assert 2 ** 62 - 2 ** 8 <= m < 2 ** 63 + 2 ** 32, v
