@@ -239,17 +239,20 @@ __global__ void __launch_bounds__(GramCfg<KIND>::kThreads, 1)
     // split x = hi + lo, hi the TF32 value the tensor core takes from x, lo = x - hi exact. A's
     // parts go to tensor memory (thread = row = lane), so that the twelve MMAs of a k-block read
     // only B from shared memory: staged A tiles and low parts were read twelve times over there,
-    // 250 bytes a clock with the loads and the split: 5.44 -> 4.93 ms at 8192 x 16640, 172.9 ->
+    // 250 bytes a clock with the loads and the split: 5.44 -> 4.97 ms at 8192 x 16640, 172.9 ->
     // 161.7 at 32768 x 34944. (Without any split work it takes 4.46: the MMAs of N = 128 themselves,
-    // about 105 clocks each, bound it now.) B's staged words are its high parts as they are (the tensor core ignores the 13 low mantissa bits); its low parts
-    // are written beside them in the same swizzled layout
+    // about 105 clocks each, bound it now.) B's staged words are its high parts as they are (the
+    // tensor core ignores the 13 low mantissa bits); its low parts are written beside them in the same
+    // swizzled layout
     const int t = threadIdx.x - 192, q = warp & 3, row = 32 * q + lane;
-    for (int64_t kb = 0; kb < nkb && !*fail; ++kb) {
+    for (int64_t kb = 0; kb < nkb; ++kb) {
       const int s = (int)(kb % kStages);
-      if (!mbar_wait(&full[s], (uint32_t)((kb / kStages) & 1))) {
+      // whole warps go on or leave: the tensor-memory stores take all 32 lanes
+      if (!__all_sync(0xffffffffu, !*fail && mbar_wait(&full[s], (uint32_t)((kb / kStages) & 1)))) {
         *fail = 1;
         break;
       }
+      tc_fence_after();  // the MMAs that read the slot's tensor memory came before this stage's load
       uint8_t* stage = smem + s * kStageBytes;
       float hi[32], lo[32];
 #pragma unroll
