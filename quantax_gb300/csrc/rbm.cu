@@ -937,6 +937,10 @@ constexpr int threads_for() {
   return JT <= 2 ? 1024 : (JT == 4 ? 512 : 256);
 }
 
+// Scratch of a warp in shared memory: a sweep keeps its configuration there, local energies keep theirs
+// in the lanes
+constexpr int kSweepWarpFloats = 32, kElocWarpFloats = 0;
+
 // Shared-memory plan: stage `stage_floats` when it fits next to the per-warp scratch.
 inline bool fits_smem(int nthreads, int64_t stage_floats, int64_t per_warp_floats, size_t* bytes) {
   const int64_t extra = per_warp_floats * (nthreads / 32) * 4;
@@ -978,7 +982,7 @@ int launch_sweep(const float* table, int n, int mp, uint32_t* spins, float* log_
                  int nsteps, uint64_t seed, uint64_t step0, float reweight, int proposal, const int32_t* nbr, int z,
                  int hop, cudaStream_t st) {
   size_t smem;
-  const bool sm = fits_smem(threads_for<JT>(), table_floats(n, mp), 32, &smem);
+  const bool sm = fits_smem(threads_for<JT>(), table_floats(n, mp), kSweepWarpFloats, &smem);
   if (proposal == QGX_PROPOSAL_LOCAL_FLIP) {
     return sm ? launch_sweep_v<JT, true, QGX_PROPOSAL_LOCAL_FLIP>(table, n, mp, spins, log_psi, accepts, ns, nsteps,
                                                                   seed, step0, reweight, nbr, z, hop, smem, st)
@@ -1011,7 +1015,7 @@ int launch_eloc(const float* table, int n, int mp, const qgx_operator_t& op, con
   constexpr int NS = JT <= 4 ? 2 : 1;
   const bool two = ns > (int64_t)device_sm_count() * (NT / 32);
   size_t smem;
-  if (fits_smem(NT, table_floats(n, mp), 32, &smem))
+  if (fits_smem(NT, table_floats(n, mp), kElocWarpFloats, &smem))
     return two ? launch_eloc_v<JT, true, NS>(table, n, mp, op, spins, ns, eloc, smem, st)
                : launch_eloc_v<JT, true, 1>(table, n, mp, op, spins, ns, eloc, smem, st);
   return two ? launch_eloc_v<JT, false, NS>(table, n, mp, op, spins, ns, eloc, smem, st)
@@ -1127,7 +1131,7 @@ int launch_sweep_batch(const qgx_rbm_sweep_job_t* jobs, const int* idx, int cnt,
     const qgx_rbm_sweep_job_t& J = jobs[idx[q]];
     const int mp = padded_m(J.m);
     size_t bytes;
-    fits_smem(NT, table_floats(J.n, mp), 32, &bytes);
+    fits_smem(NT, table_floats(J.n, mp), kSweepWarpFloats, &bytes);
     smem = std::max(smem, bytes);
     b.job[q] = SweepJob{J.table, J.spins, J.log_psi, J.accepts, J.nbr, J.ns, table_floats(J.n, mp), J.seed, J.step0,
                         J.reweight, J.n, mp, J.nsteps, J.z, J.hop};
@@ -1152,7 +1156,7 @@ int launch_eloc_batch(const qgx_rbm_eloc_job_t* jobs, const int* idx, int cnt, c
     const qgx_rbm_eloc_job_t& J = jobs[idx[q]];
     const int mp = padded_m(J.m);
     size_t bytes;
-    fits_smem(NT, table_floats(J.n, mp), 32, &bytes);
+    fits_smem(NT, table_floats(J.n, mp), kElocWarpFloats, &bytes);
     smem = std::max(smem, bytes);
     b.job[q] = ElocJob{*J.op, J.table, J.spins, J.eloc, J.ns, table_floats(J.n, mp), J.n, mp};
     ns[q] = J.ns;
@@ -1183,11 +1187,12 @@ int eloc_batch_jt(const qgx_rbm_eloc_job_t* jobs, const int* idx, int cnt, bool 
   return sm ? launch_eloc_batch<JT, true>(jobs, idx, cnt, st) : launch_eloc_batch<JT, false>(jobs, idx, cnt, st);
 }
 
-// whether job (n, mp)'s table is staged in shared memory by the kernels of width JT
-inline bool stages_in_smem(int jt, int n, int mp) {
+// whether job (n, mp)'s table is staged in shared memory by the kernels of width JT, beside
+// per_warp_floats of scratch
+inline bool stages_in_smem(int jt, int n, int mp, int per_warp_floats) {
   size_t bytes;
   const int nt = jt <= 2 ? 1024 : (jt == 4 ? 512 : 256);  // threads_for<JT>()
-  return fits_smem(nt, table_floats(n, mp), 32, &bytes);
+  return fits_smem(nt, table_floats(n, mp), per_warp_floats, &bytes);
 }
 
 }  // namespace
@@ -1316,7 +1321,7 @@ int qgx_rbm_sweep_batched(const qgx_rbm_sweep_job_t* jobs, int32_t njobs, int32_
     QGX_CHECK_ARG(J.table && J.spins && J.log_psi);
     const int mp = padded_m(J.m);
     if (!mp_supported(mp)) return QGX_ERR_UNSUPPORTED;
-    cls[j] = BatchClass{mp / 128, stages_in_smem(mp / 128, J.n, mp) ? 1 : 0, J.proposal};
+    cls[j] = BatchClass{mp / 128, stages_in_smem(mp / 128, J.n, mp, kSweepWarpFloats) ? 1 : 0, J.proposal};
     live[j] = true;
   }
   const cudaStream_t st = as_cuda(stream);
@@ -1358,7 +1363,7 @@ int qgx_rbm_eloc_batched(const qgx_rbm_eloc_job_t* jobs, int32_t njobs, int32_t*
     QGX_CHECK_ARG(J.table && J.spins && J.eloc);
     const int mp = padded_m(J.m);
     if (!mp_supported(mp)) return QGX_ERR_UNSUPPORTED;
-    cls[j] = BatchClass{mp / 128, stages_in_smem(mp / 128, J.n, mp) ? 1 : 0, 0};
+    cls[j] = BatchClass{mp / 128, stages_in_smem(mp / 128, J.n, mp, kElocWarpFloats) ? 1 : 0, 0};
     live[j] = true;
   }
   const cudaStream_t st = as_cuda(stream);
