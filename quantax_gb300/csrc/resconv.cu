@@ -152,7 +152,9 @@ __device__ inline void fma_pair(float2& c, float2 a, float2 b) {
 // sites as such addresses, so that a gather is one 32-bit addition (of the input channel's offset)
 // and a load; through 64-bit pointers the compiler's address arithmetic took issue slots and
 // registers from the multiply-adds (2.58 against 2.44 ms per 16384 forwards at L = 10, 8 blocks,
-// 16 channels).
+// 16 channels). The compiler does not know what it reads: a convolution's loads stand between two
+// order_shared, which no load or store of the code around passes.
+__device__ inline void order_shared() { asm volatile("" ::: "memory"); }
 __device__ inline float ld_shared(uint32_t addr) {
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
@@ -170,6 +172,7 @@ __device__ inline void conv_layer(const float* __restrict__ in, int cin, float* 
                                   int mode, int ss) {  // ss: floats between samples' activations
   const float* bias = w + cin * 9 * C;
   const int G = (N + SPT - 1) / SPT;
+  order_shared();
   for (int it = threadIdx.x; it < S * G; it += blockDim.x) {
     const int a = it / G, g = it - a * G;
     int r[SPT];
@@ -228,6 +231,7 @@ __device__ inline void conv_layer(const float* __restrict__ in, int cin, float* 
       }
     }
   }
+  order_shared();
 }
 
 // out[a][o][b] = act(sum_{i,tap} W[i][tap][o] in[a][i][b + tap] + bias[o]) in the blocked site
@@ -257,6 +261,7 @@ __device__ inline void conv_layer_blocked(const float* __restrict__ in, int cin_
   const int NB = N >> 2;
   const int items = S * NB;
   const int per = (items + 31) & ~31;  // items of one channel group, rounded to whole warps
+  order_shared();
   for (int it = threadIdx.x; it < H * per; it += blockDim.x) {
     const int h = it / per, j = it - h * per;
     if (j >= items) continue;
@@ -322,6 +327,7 @@ __device__ inline void conv_layer_blocked(const float* __restrict__ in, int cin_
       }
     }
   }
+  order_shared();
 }
 
 // 4 x 4 input patches of the 2 x 2 blocks (rows 2 by - 1 .. 2 by + 2, columns 2 bx - 1 .. 2 bx + 2,
