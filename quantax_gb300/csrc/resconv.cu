@@ -599,8 +599,7 @@ __global__ void rc_set_step_kernel(uint64_t* __restrict__ step_base, uint64_t st
 
 // One warp per sample, its connected configurations over the lanes (fixed order: lane, then the
 // warp's sum tree): the FP64 exponentials and sines are what it costs, and a thread per sample left
-// most of the FP64 pipes idle (1024
-// samples of 205 configurations: about 600 us, now 37).
+// most of the FP64 pipes idle (1024 samples of 205 configurations: about 600 us, now 37).
 __global__ void rc_eloc_reduce_kernel(qgx_operator_t op, const uint32_t* __restrict__ spins, int64_t ns, int n,
                                       const float2* __restrict__ lp, const int64_t* __restrict__ offsets,
                                       const double* __restrict__ elem, const float2* __restrict__ lp_conn,
@@ -618,8 +617,9 @@ __global__ void rc_eloc_reduce_kernel(qgx_operator_t op, const uint32_t* __restr
     const float2 l = lp_conn[k];
     const double m = exp((double)l.x - (double)l0.x);
     const double ph = (double)l.y - (double)l0.y;
-    if (ph == 0.0) {  // real amplitudes of one sign
+    if (ph == 0.0) {  // real amplitudes of one sign: cosine 1, sine 0
       re += elem[k] * m;
+      if (ei) im += elem[k] * m * ph;  // not a number where the ratio is none or overflows
       continue;
     }
     double sn, cs;
