@@ -140,14 +140,14 @@ __global__ void __launch_bounds__(kWeakThreads)
   while (bi * (bi + 1) / 2 > tile) --bi;
   const int64_t r0 = bi * kWeakTile, c0 = (tile - bi * (bi + 1) / 2) * kWeakTile;
   constexpr int kWarps = kWeakThreads / 32, kRows = kWeakTile / kWarps;  // rows per warp
-  uint32_t hi[kRows][2];  // high words, the sign out; 1 for a value that only the low word holds
+  uint32_t hi[kRows][2];  // exponent and leading bits, the sign out; 1 for a value that only later bits hold
 #pragma unroll
   for (int k = 0; k < kRows; ++k)
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const int64_t r = r0 + warp + k * kWarps, j = c0 + 32 * q + lane;
       const uint64_t b = r < n && j < r ? dbl_bits(A[r * lda + j]) << 1 : 0;
-      hi[k][q] = (uint32_t)(b >> 33) | ((uint32_t)b != 0);
+      hi[k][q] = (uint32_t)(b >> 33) | (b << 31 != 0);
     }
   if (t < kWeakTile) {
     er[t] = r0 + t < n ? row_exponent(bound, r0 + t) : 0;

@@ -56,6 +56,19 @@ def test_weak_couplings(cuda, n, c):
     check(coupled(n, c, n))
 
 
+@pytest.mark.parametrize("bit", [0, 30, 31, 32, 51, 52])
+def test_smallest_couplings(cuda, bit):
+    """One bit of the value set: subnormal couplings, and the smallest normal one."""
+    n = 70
+    c = 2.0 ** (bit - 1074)
+    A = torch.full((n, n), c, dtype=torch.float64, device="cuda")
+    A.diagonal().fill_(1.0)
+    assert factor(A) == 0
+    want = torch.full((n, n), c, dtype=torch.float64, device="cuda")
+    want.diagonal().fill_(1.0)
+    assert torch.equal(A, want)
+
+
 @pytest.mark.parametrize("scales", [300])
 def test_weak_couplings_scaled_rows(cuda, scales):
     A = coupled(130, 1e-6, 7)
