@@ -69,9 +69,9 @@ FORMS = {
 # DRAM bytes per Gram launch at the bench's shapes (profiles/gram_tc_3xtf32_rows8192_k16640.md):
 #   ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum --clock-control none \
 #       -k regex:gram_tc -s 2 -c 1 python -m quantax_gb300.kernel_bench gram --mode 3xtf32 --rows 8192 --k 16640 --reps 1
-# rbm (8192 x 16640): 5.42 GB read + 0.51 GB written. resconv (32768 x 34944): the capture at 8192 rows x
-# 34944 (11.38 + 0.51 GB) scaled by (32768 / 8192)^2, the growth of the tile pairs that re-read the operand.
-GRAM_TRAFFIC_BYTES = {("rbm", "3xtf32"): 4.30e9, ("resconv", "3xtf32"): 4 * (32.79e9 + 2.14e9)}
+# rbm (8192 x 16640): 3.78 GB read + 0.52 GB written. resconv (32768 x 34944): the capture at 16384 rows x
+# 34944 (45.70 + 2.15 GB) scaled by (32768 / 16384)^2, the growth of the tile pairs that re-read the operand.
+GRAM_TRAFFIC_BYTES = {("rbm", "3xtf32"): 4.30e9, ("resconv", "3xtf32"): 4 * (45.70e9 + 2.15e9)}
 
 
 def peaks():

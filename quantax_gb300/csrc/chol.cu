@@ -777,7 +777,8 @@ constexpr int chain_threads(int tiles) { return std::max(kPotrfThreads, 32 * (kT
 // the trailing update that runs beside, so this is for rows that leave it some; one tile per CTA, with
 // no other tile's integer work beside the chain, where there are few. About 50 us a block with the
 // update of the next columns (62 as two launches): n = 1056: 1.06 -> 0.87 ms, 4096: 4.36 -> 3.63, 8192:
-// 11.5 -> 10.5.
+// 11.5 -> 10.5. Jobs on other streams do not pay for it: eight served together run at 96.4 steps/s, 94.6
+// with two launches.
 template <int TILES>
 __global__ void __launch_bounds__(chain_threads(TILES), 1)
     chain_block_kernel(double* __restrict__ A, int64_t lda, int64_t c, int nb, int64_t n, RowBound bound,
@@ -958,8 +959,8 @@ __device__ inline bool oz_tile(int64_t index, int64_t m, int64_t ncols, int64_t*
 // a persistent grid: the panel chain of the look-ahead runs beside this kernel and gets an SM only
 // when a CTA ends. Measured: 1.67 ms for the 15872-row update of a 16384 factorisation, tensor pipe
 // 59% (31.5% for 128 x 32 tiles, two CTAs per SM, single 80 KB stages, 36 products of N = 32 ..
-// 256); the rest is the drain of the accumulators between tiles and the first and last tile of a
-// CTA. The factorisation at n = 32768: 342 ms, 617 before.
+// 256); L2 runs at a quarter of its rate, so the rest is most likely the drain of the accumulators between
+// tiles and the first and last tile of a CTA. The factorisation at n = 32768: 343 ms, 617 before.
 __global__ void __launch_bounds__(kOzThreads, 1)
     ozaki_syrk_kernel(const uint8_t* __restrict__ S, const int* __restrict__ ex, int kblocks, int off, int64_t m,
                       int64_t ncols, double* __restrict__ C, int64_t ldc, int64_t tiles, int per_cta,

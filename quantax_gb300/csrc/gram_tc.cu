@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(GramCfg<KIND>::kThreads, 1)
     // split x = hi + lo, hi the TF32 value the tensor core takes from x, lo = x - hi exact. A's
     // parts go to tensor memory (thread = row = lane), so that the twelve MMAs of a k-block read
     // only B from shared memory: staged A tiles and low parts were read twelve times over there,
-    // 250 bytes a clock with the loads and the split: 5.44 -> 4.97 ms at 8192 x 16640, 172.9 ->
+    // 250 bytes a clock with the loads and the split: 5.44 -> 4.95 ms at 8192 x 16640, 172.9 ->
     // 161.7 at 32768 x 34944. (Without any split work it takes 4.46: the MMAs of N = 128 themselves,
     // about 105 clocks each, bound it now.) B's staged words are its high parts as they are (the
     // tensor core ignores the 13 low mantissa bits); its low parts are written beside them in the same
