@@ -127,53 +127,76 @@ __global__ void diag_bound_kernel(const double* __restrict__ A, int64_t lda, int
 // 4.5e-17 at c = 2^-4, 7.9e-17 and 1.2e-16 at 2^-7 (a tenth of the entries weak), 7.7e-17 and 2.4e-16 at
 // 2^-8 (a fifth, of some row more than a quarter), 7.5e-17 and 9.7e-13 at 2^-20. Of a Gram of RBM or
 // ResConv samples 1 to 5% are weak (13% in a row of 6000 samples of 65536 parameters).
-// One pass over the lower triangle: 8 us of 0.90 ms at n = 1056, 0.1 of 10.7 ms at 8192.
+// One pass over the lower triangle, bound by the latency of its loads: a CTA walks along a row of tiles
+// and loads the next one beside the count (n = 1056: 5 us, 8192: 53 us; 101 with a CTA per tile).
 constexpr int kWeakBits = 12, kWeakTile = 64, kWeakThreads = 256;
 __global__ void __launch_bounds__(kWeakThreads)
-    weak_coupling_kernel(const double* __restrict__ A, int64_t lda, int64_t n, RowBound bound, int* __restrict__ score) {
-  __shared__ int er[kWeakTile], ec[kWeakTile], col_score[kWeakTile];
+    weak_coupling_kernel(const double* __restrict__ A, int64_t lda, int64_t n, RowBound bound, int per_cta,
+                         int* __restrict__ score) {
+  // row tile blockIdx.y, per_cta column tiles from blockIdx.x per_cta on
+  const int64_t first = blockIdx.x * (int64_t)per_cta, last = min(first + per_cta, (int64_t)blockIdx.y + 1);
+  if (first >= last) return;
+  __shared__ int er[kWeakTile], ec[2][kWeakTile], col_score[2][kWeakTile];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  // lower-triangular tile index -> (bi, bj), bi >= bj
-  const int64_t tile = blockIdx.x;
-  int64_t bi = (int64_t)((sqrtf(8.0f * (float)tile + 1.0f) - 1.0f) * 0.5f);
-  while ((bi + 1) * (bi + 2) / 2 <= tile) ++bi;
-  while (bi * (bi + 1) / 2 > tile) --bi;
-  const int64_t r0 = bi * kWeakTile, c0 = (tile - bi * (bi + 1) / 2) * kWeakTile;
+  const int64_t r0 = blockIdx.y * (int64_t)kWeakTile;
   constexpr int kWarps = kWeakThreads / 32, kRows = kWeakTile / kWarps;  // rows per warp
-  uint32_t hi[kRows][2];  // exponent and leading bits, the sign out; 1 for a value that only later bits hold
+  double v[kRows][2];
+  int e = 0;  // exponent of column t
+  auto load = [&](int64_t tile) {
+    const int64_t c0 = tile * kWeakTile;
 #pragma unroll
-  for (int k = 0; k < kRows; ++k)
+    for (int k = 0; k < kRows; ++k)
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int64_t r = r0 + warp + k * kWarps, j = c0 + 32 * q + lane;
-      const uint64_t b = r < n && j < r ? dbl_bits(A[r * lda + j]) << 1 : 0;
-      hi[k][q] = (uint32_t)(b >> 33) | (b << 31 != 0);
-    }
+      for (int q = 0; q < 2; ++q) {
+        const int64_t r = r0 + warp + k * kWarps, j = c0 + 32 * q + lane;
+        v[k][q] = r < n && j < r ? A[r * lda + j] : 0.0;
+      }
+    if (t < kWeakTile && c0 + t < n) e = row_exponent(bound, c0 + t);
+  };
+  load(first);
   if (t < kWeakTile) {
     er[t] = r0 + t < n ? row_exponent(bound, r0 + t) : 0;
-    ec[t] = c0 + t < n ? row_exponent(bound, c0 + t) : 0;
-    col_score[t] = 0;
+    col_score[0][t] = col_score[1][t] = 0;
   }
-  __syncthreads();
-  int cs[2] = {};  // scores: 3 for a weak entry, -1 for another that is not zero
+  int rs[kRows] = {};  // scores: 3 for a weak entry, -1 for another that is not zero
+  for (int64_t tile = first; tile < last; ++tile) {
+    const int buf = (int)(tile & 1);
+    uint32_t hi[kRows][2];  // exponent and leading bits, the sign out; 1 for a value that only later bits hold
+#pragma unroll
+    for (int k = 0; k < kRows; ++k)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint64_t b = dbl_bits(v[k][q]) << 1;
+        hi[k][q] = (uint32_t)(b >> 33) | (b << 31 != 0);
+      }
+    if (t < kWeakTile) ec[buf][t] = e;
+    if (tile + 1 < last) load(tile + 1);
+    __syncthreads();
+    const int limit[2] = {ec[buf][lane] - kWeakBits + 1022, ec[buf][32 + lane] - kWeakBits + 1022};
+    int cs[2] = {};
+#pragma unroll
+    for (int k = 0; k < kRows; ++k)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        // |a| < 2^(exponent field - 1022)
+        const int s = hi[k][q] == 0 ? 0 : (int)(hi[k][q] >> 20) <= er[warp + k * kWarps] + limit[q] ? 3 : -1;
+        rs[k] += s;
+        cs[q] += s;
+      }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) atomicAdd(&col_score[buf][32 * q + lane], cs[q]);
+    __syncthreads();
+    if (t < kWeakTile) {
+      const int64_t c = tile * kWeakTile + t;
+      if (col_score[buf][t] != 0) atomicAdd(score + c, col_score[buf][t]);
+      col_score[buf][t] = 0;  // used again two tiles on
+    }
+  }
 #pragma unroll
   for (int k = 0; k < kRows; ++k) {
-    const int i = warp + k * kWarps;
-    int rs = 0;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      // |a| < 2^(exponent field - 1022)
-      const int s = hi[k][q] == 0 ? 0 : (int)(hi[k][q] >> 20) - 1022 <= er[i] + ec[32 * q + lane] - kWeakBits ? 3 : -1;
-      rs += s;
-      cs[q] += s;
-    }
-    rs = __reduce_add_sync(0xffffffffu, rs);
-    if (lane == 0 && rs != 0) atomicAdd(score + r0 + i, rs);
+    const int s = __reduce_add_sync(0xffffffffu, rs[k]);
+    if (lane == 0 && s != 0) atomicAdd(score + r0 + warp + k * kWarps, s);
   }
-#pragma unroll
-  for (int q = 0; q < 2; ++q) atomicAdd(&col_score[32 * q + lane], cs[q]);
-  __syncthreads();
-  if (t < kWeakTile && col_score[t] != 0) atomicAdd(score + c0 + t, col_score[t]);
 }
 
 constexpr int kChooseThreads = 1024;
@@ -1275,14 +1298,16 @@ int chol_f64(double* A, int64_t n, int64_t lda, int* info, int32_t* status, void
                                       (int)sizeof(TrsmShared<1>)));
   int* score = ws.e_panel[1];  // free until the second panel is sliced
   diag_bound_kernel<<<(unsigned)((n + 255) / 256), 256, 0, aux>>>(A, lda, n, ws.bound, ws.chain, score, info);
-  const int64_t scans = (n + kWeakTile - 1) / kWeakTile, scan_tiles = scans * (scans + 1) / 2;
-  if (scan_tiles > 0x7fffffffLL) return QGX_ERR_UNSUPPORTED;
-  weak_coupling_kernel<<<(unsigned)scan_tiles, kWeakThreads, 0, aux>>>(A, lda, n, ws.bound, score);
+  // column tiles per CTA: one where that leaves SMs idle, else up to eight, whose loads overlap
+  const int64_t scans = (n + kWeakTile - 1) / kWeakTile, sms = device_sm_count();
+  const int scan_per = (int)std::max<int64_t>(1, std::min<int64_t>(8, scans * (scans + 1) / 2 / (4 * sms)));
+  if (scans > 65535) return QGX_ERR_UNSUPPORTED;
+  weak_coupling_kernel<<<dim3((unsigned)((scans + scan_per - 1) / scan_per), (unsigned)scans), kWeakThreads, 0, aux>>>(
+      A, lda, n, ws.bound, scan_per, score);
   choose_panel_kernel<<<1, kChooseThreads, 0, aux>>>(score, n, ws.chain);
   *kernels += 3;
   int64_t k = 0;
   unsigned tickets = 0;  // drawn by the launches so far
-  const int64_t sms = device_sm_count();
   for (int64_t c0 = 0; c0 < n; c0 += kPanel, ++k) {
     const int64_t pe = std::min<int64_t>(c0 + kPanel, n);
     if (k >= 2) QGX_CHECK_CUDA(cudaStreamWaitEvent(aux, la->rest_done[k & 1], 0));

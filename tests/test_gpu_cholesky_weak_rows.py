@@ -104,6 +104,26 @@ def test_weak_couplings_in_every_launch_form(cuda, n):
     assert bool(((L.diagonal() - 1.0).abs() <= 2.0 ** -52).all())
 
 
+@pytest.mark.parametrize("n", [700, 4500, 7500])
+@pytest.mark.parametrize("where", [0.0, 0.0143, 0.5, 0.99, 1.0])
+def test_one_weak_row_is_found(cuda, n, where):
+    """Couplings of 2^-8 everywhere, of 2^-30 in one row and column: fixed point would keep their
+    products to about 2^-61, FP64 to n 2^-83."""
+    k = int(where * (n - 1))
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    S = (torch.randint(0, 2, (n, n), generator=g, device="cuda", dtype=torch.int8).double() * 2 - 1).tril(-1) * 2.0 ** -8
+    A = S + S.T
+    w = (1.0 + torch.rand(n, generator=g, device="cuda", dtype=torch.float64)) * 2.0 ** -30
+    A[k], A[:, k] = w, w
+    A.diagonal().fill_(1.0)
+    L = A.clone()
+    assert factor(L) == 0
+    L = L.tril()
+    err = (L @ L[k] - A[k]).abs()
+    err[k] = 0.0
+    assert float(err.max()) <= 2.0 ** -66
+
+
 @pytest.mark.parametrize("n,row", [(64, 40), (300, 200), (300, 5), (7500, 7000)])
 def test_minor_that_fails_among_weak_rows(cuda, n, row):
     A = torch.as_tensor(coupled(n, 1e-6, 3) if n < 1000 else np.diag(np.ones(n)) + 1e-6 * (1 - np.eye(n))).cuda()
